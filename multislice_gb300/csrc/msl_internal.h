@@ -1,6 +1,7 @@
 // Internal host-side interface between the C ABI (msl_api.cu) and the kernels.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -172,6 +173,11 @@ float k2max_f32(int nx, int ny, double ax, double by, double bw);
 void prop_tables(int nx, int ny, const msl_optics *o, double dz, const float *kx, const float *kx2,
                  const float *ky, const float *ky2, float2 *px, float2 *py);
 
+// A tiled tensor map (strides in bytes, of dimensions 1..rank-1); false where the
+// driver entry point is missing or refuses it.
+bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const uint64_t *dims,
+                       const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle);
+
 // Each launcher returns cudaSuccess or the launch error; *launches is bumped.
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, int64_t *launches);
@@ -266,21 +272,20 @@ int resident_cluster();
 struct ClosureNet {
     float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
     __nv_bfloat16 *wt = nullptr;      // expanded bf16 weights of the tensor-core layers
-    float *dwreal = nullptr;          // one layer's real weight gradient + bias gradient
     void *acts = nullptr;             // activations
     float *partial = nullptr;         // weight-gradient partial sums
     double *loss_part = nullptr;      // per-block loss sums
+    double *rms_part = nullptr;       // per-block sums of |psi|^2
     float *scale = nullptr;           // per-image s and 1/s
-    size_t cap_pix = 0;
+    size_t cap_bytes = 0, cap_pix = 0;
     int cap_img = 0;
-    bool cap_train = false;
     int step = 0;
     int loss_blocks = 0;
     __nv_bfloat16 *hbuf[6] = {}, *dh[2] = {}, *xbuf = nullptr;
     float *g6 = nullptr;
     cudaError_t alloc_params();
     void release();
-    cudaError_t ensure(size_t npix, int nimg, bool train);
+    cudaError_t ensure(int B, int H, int W, bool train);
     cudaError_t expand(cudaStream_t s, int nsm, int64_t *launches);
     cudaError_t conv_tc(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
                         const __nv_bfloat16 *mask, __nv_bfloat16 *out, int B, int H, int W, int epi, int *err,

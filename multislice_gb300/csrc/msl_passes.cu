@@ -1375,6 +1375,15 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
+bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const uint64_t *dims,
+                       const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle) {
+    if (!encode_fn()) return false;
+    const cuuint32_t estride[3] = {1, 1, 1};
+    return encode_fn()(map, type, (cuuint32_t)rank, (void *)base, (const cuuint64_t *)dims, (const cuuint64_t *)strides,
+                       box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // The TMA kernel needs one buffer for load and store (in place) at a 16-byte
 // aligned address; other calls take the register-only kernel.
 static bool tma_eligible(const ColArgs &a) {

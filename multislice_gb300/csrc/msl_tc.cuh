@@ -46,6 +46,16 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
            | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
 
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// What N columns add to an instruction descriptor.
+__host__ __device__ constexpr uint32_t idesc_n(int N) { return (uint32_t)(N >> 3) << 17; }
+
 // TMEM allocation by one full warp; the base address is written to *dst (shared).
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
@@ -108,6 +118,24 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 64 consecutive FP32 columns of this thread's TMEM lane: four loads, one wait.
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
+    uint32_t r[64];
+#pragma unroll
+    for (int q = 0; q < 64; q += 16)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15}, [%16];"
+            : "=r"(r[q]), "=r"(r[q + 1]), "=r"(r[q + 2]), "=r"(r[q + 3]), "=r"(r[q + 4]), "=r"(r[q + 5]),
+              "=r"(r[q + 6]), "=r"(r[q + 7]), "=r"(r[q + 8]), "=r"(r[q + 9]), "=r"(r[q + 10]), "=r"(r[q + 11]),
+              "=r"(r[q + 12]), "=r"(r[q + 13]), "=r"(r[q + 14]), "=r"(r[q + 15])
+            : "r"(taddr + (uint32_t)q)
+            : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 }  // namespace tc

@@ -96,3 +96,23 @@ def test_closure_gain_on_held_out_srtio3_probes(ctx):
     net.close()
     del coarse, fine
     torch.cuda.empty_cache()
+
+
+# one row less than a tile needs, strips that split unevenly, several strips a
+# row, and more strips than the GPU has SMs (a CTA then walks several)
+@pytest.mark.parametrize("B,H,W", [(1, 3, 128), (2, 37, 256), (1, 5, 384), (170, 3, 128)])
+def test_closure_shapes_match_oracle(ctx, B, H, W):
+    from multislice_gb300.api import Closure
+    net = Closure(ctx, seed=7)
+    p = CO.init_params(13, scale_last=1.0)
+    net.set_params(p)
+    c, f = _waves(B + H + W, B, H, W)
+    loss, g = net.gradients(c, f)
+    got = net.apply(c.copy())
+    ref, _, _ = CO.forward(p, c, bf=True)
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref - c) < 1e-3
+    ref_loss, ref_g = CO.gradient(p, c, f, bf=True)
+    assert abs(loss - ref_loss) <= 1e-4 * ref_loss
+    for l, sl in enumerate(_layer_slices()):
+        assert np.linalg.norm(g[sl] - ref_g[sl]) / np.linalg.norm(ref_g[sl]) < 2e-2, l
+    net.close()
