@@ -1501,6 +1501,7 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
             none.d_prop = nullptr;
             ColArgs pa = col_args(&jb.grid, none, g.twc, 0, slot, 1, msl::COL_PROBE | msl::COL_INV | msl::COL_STORE,
                                   c->dflag);
+            pa.shared = concurrent;
             pa.apchi = apchi;
             pa.ex = ex;
             pa.ey = ey;
@@ -1518,15 +1519,18 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
             RowArgs r = row_args(&gg, g.twr, nullptr, w, nact,
                                  msl::ROW_LOAD | msl::ROW_INV | msl::ROW_TRANS | msl::ROW_FWD, c->dflag);
             r.trans_b = ttab + (size_t)s * nb;
+            r.shared = concurrent;
             LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, st, c->nsm, &c->launches); }));
             ColArgs ca = col_args(&gg, none, g.twc, 0, w, nact,
                                   msl::COL_LOAD | msl::COL_FWD | msl::COL_PROP | msl::COL_INV | msl::COL_STORE, c->dflag);
+            ca.shared = concurrent;
             ca.prop_b = ptabd + (size_t)s * nb;
             ca.k2_b = ktab;
             ca.k2max_b = dk2max;
             LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, st, c->nsm, &c->launches); }));
         }
         RowArgs r = row_args(&gg, g.twr, nullptr, w, nb, msl::ROW_LOAD | msl::ROW_INV, c->dflag);
+        r.shared = concurrent;
         LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, st, c->nsm, &c->launches); }));
         if (concurrent) {
             cudaEvent_t e = take_event(c);

@@ -74,6 +74,7 @@ struct RowArgs {
     double *accum;         // [nlines][ny] (ROW_ACCUM)
     double accum_w;
     const float2 *const *trans_b;  // per-image transmission rows (replaces trans when set)
+    bool shared;           // other streams' kernels run beside this one
 };
 
 // Column pass: strided lines of length nx (one line = one iy of one image).
@@ -110,6 +111,7 @@ struct ColArgs {
     const float2 *const *prop_b;
     const float *const *k2_b;
     const float *k2max_b;
+    bool shared;              // other streams' kernels run beside this one
 };
 
 struct PotArgs {
