@@ -184,6 +184,14 @@ bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, con
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches);
+// One propagator table: float frequencies kx[nx] then ky[ny] (device), slice
+// thickness, wavelength and 2 tan(tilt); out[ntab][nx + ny].  Part of a call's set-up
+// like its uploads: not counted as a launch.
+struct PropTable {
+    const float *k;
+    double dz, lam, ttx, tty;
+};
+cudaError_t launch_prop_tables(const PropTable *tabs, int ntab, int nx, int ny, float2 *out, cudaStream_t s);
 // apchi[ix][iy] = A(s) exp(-i chi(s)) * scale, s = kx^2 + ky^2 from kxd/kyd (FP64)
 cudaError_t launch_probe_table(int nx, int ny, const double *kxd, const double *kyd, double s_in,
                                double s_out, double lam, double df, double cs, double scale,
