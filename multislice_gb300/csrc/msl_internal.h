@@ -73,6 +73,10 @@ struct RowArgs {
     int *err;              // set to 1 when a bounded wait gives up (may be null)
     double *accum;         // [nlines][ny] (ROW_ACCUM)
     double accum_w;
+    // many images onto one accumulator (ROW_LOAD [| ROW_INV] | ROW_ACCUM | ROW_NOSTORE):
+    // image i of nimg adds accum_wt[(img0 + i) % nw] * |psi|^2 to accum[nx][ny], in order
+    int nimg, img0, nw;        // nimg = 0: one image per accumulator, accum_w
+    const double *accum_wt;
     const float2 *const *trans_b;  // per-image transmission rows (replaces trans when set)
     bool shared;           // other streams' kernels run beside this one
 };
@@ -106,6 +110,9 @@ struct ColArgs {
     double *partial;          // [batch][ny / C][ndet]
     int *err;                 // set to 1 when a bounded wait gives up (may be null)
     const float2 *ctf;        // [nx][ny] (COL_CTF)
+    // several results per image: result b of the batch is image (img0 + b) / fan of `in`
+    // times ctf[(img0 + b) % fan], stored to image b of `out` (fan = 0: in place, one ctf)
+    int fan, img0;
     // per-image tables (replace px/py, kx2/ky2, k2max when set): prop_b[b] -> px[nx] py[ny],
     // k2_b[b] -> kx2[nx] ky2[ny], k2max_b[b]
     const float2 *const *prop_b;
@@ -204,15 +211,15 @@ cudaError_t launch_detector_mask(int nx, int ny, const double *kxd, const double
                                  const double *kin2, const double *kout2, uint8_t *mask,
                                  cudaStream_t s, int64_t *launches);
 // ctf[ix][iy] = exp(-i chi(k)) * scale for k2 = kx2 + ky2 (float) <= k2obj, else 0;
-// chi = pi lam k2 (cs lam^2 k2 / 2 - df) in FP64
+// chi = pi lam k2 (cs lam^2 k2 / 2 - df) in FP64, one table per defocus value df[ndf] (device)
 struct CtfParams {
-    double lam, cs, df, dfa2, dfa2phi, dfa3, dfa3phi;
+    double lam, cs, dfa2, dfa2phi, dfa3, dfa3phi;
     float k2obj, scale;
 };
 // phi = atan2(ky, kx) from the float kx / ky tables (astigmatism terms)
 cudaError_t launch_ctf_table(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
-                             const float *ky, const CtfParams &p, float2 *ctf, cudaStream_t s,
-                             int64_t *launches);
+                             const float *ky, const CtfParams &p, const double *df, int ndf, float2 *ctf,
+                             cudaStream_t s, int64_t *launches);
 // out[b][ix][iy] = exp(2 pi i (qx[b] xpos[ix] + qy[b] ypos[iy])), the sum in float as mulslice.cpp:573-577
 cudaError_t launch_tilt_waves(int nx, int ny, int nb, const float *xpos, const float *ypos,
                               const float *q, float2 *out, cudaStream_t s, int64_t *launches);

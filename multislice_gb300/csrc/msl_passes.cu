@@ -87,8 +87,30 @@ __device__ __forceinline__ int spread_id(int w, int n, bool shared) {
     return shared ? (int)blockIdx.x * n + w : w * (int)gridDim.x + (int)blockIdx.x;
 }
 
+// One image's share of a row's running sums; acc: this thread's first element.
+template <int T, int E>
+__device__ __forceinline__ void add_image(double (&sum)[E], const float2 (&v)[E], const RowArgs &a, int img, double *acc) {
+    const double w = a.accum_wt[(a.img0 + img) % a.nw];
+    if (img == 0) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) sum[e] = acc[T * e];
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) sum[e] += w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
+    if (img == a.nimg - 1) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[T * e] = sum[e];
+    }
+}
+
 // ---------------------------------------------------------------- row pass
-template <int N>
+// IMG (this and the other row kernels; the two-stage plans have row_images_kernel): the
+// pass adds many images' intensities onto one accumulator (an image's rows through
+// many defocus values, angles or configurations), load, inverse transform and sum only.
+// A worker keeps a row's FP64 sums in registers and walks the images in order, so each
+// accumulator is read and written once per launch and the sum order does not depend
+// on how images are grouped into launches.
+template <int N, bool IMG>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS) row_pass_kernel(RowArgs a) {
     using P = Plan<N>;
     constexpr int T = P::T, E = P::E, LPB = RowCfg<N>::LPB, TW = plan_tw_size<P>();
@@ -99,10 +121,13 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) row_pass_kernel(RowArgs a)
     for (int i = tid; i < TW; i += RowCfg<N>::THREADS) tw[i] = a.tw[i];
     const int t = threadIdx.x;
     RowAddr<P> ad{lines + threadIdx.y * row_line_slots<P>()};
-    const int ngroups = (a.nlines + LPB - 1) / LPB;
+    const int ngroups = IMG ? a.nx / LPB : (a.nlines + LPB - 1) / LPB, nimg = IMG ? a.nimg : 1;
     pass_begin();
-    for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
-        const int line = g * LPB + threadIdx.y;
+    [[maybe_unused]] double sum[IMG ? E : 1];
+    for (int k = 0;; ++k) {
+        const int g = blockIdx.x + (k / nimg) * gridDim.x, img = k % nimg;
+        if (g >= ngroups) break;
+        const int line = g * LPB + threadIdx.y + img * a.nx;
         const bool valid = line < a.nlines;
         const size_t base = (size_t)line * N;
         float2 v[E];
@@ -137,7 +162,9 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) row_pass_kernel(RowArgs a)
 #pragma unroll
                 for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
             }
-            if (a.flags & ROW_ACCUM) {
+            if constexpr (IMG) {
+                add_image<T>(sum, v, a, img, a.accum + (size_t)(line % a.nx) * N + t);
+            } else if (a.flags & ROW_ACCUM) {
 #pragma unroll
                 for (int e = 0; e < E; ++e)
                     a.accum[base + t + T * e] +=
@@ -192,10 +219,13 @@ __device__ __forceinline__ void col_propagate(float2 (&v)[P::E], const ColArgs &
 
 // Objective-lens transfer of mulslice.cpp:613-633 from a precomputed table.
 template <class P>
-__device__ __forceinline__ void col_ctf(float2 (&v)[P::E], const ColArgs &a, int iy, int t) {
+__device__ __forceinline__ void col_ctf(float2 (&v)[P::E], const ColArgs &a, int b, int iy, int t) {
+    const float2 *ctf = a.ctf + (a.fan ? (size_t)((a.img0 + b) % a.fan) * P::N * a.ny : 0);
 #pragma unroll
-    for (int e = 0; e < P::E; ++e) v[e] = c_mul(v[e], a.ctf[(size_t)(t + P::T * e) * a.ny + iy]);
+    for (int e = 0; e < P::E; ++e) v[e] = c_mul(v[e], ctf[(size_t)(t + P::T * e) * a.ny + iy]);
 }
+// The image of `in` that result b of the batch starts from.
+__device__ __forceinline__ int col_source(const ColArgs &a, int b) { return a.fan ? (a.img0 + b) / a.fan : b; }
 
 // Annular detector partial sums of one tile (MSProject.cs:806-829): float per
 // thread over its E pixels, then double across the CTA in a fixed order.
@@ -253,16 +283,17 @@ __global__ void __launch_bounds__(ColCfg<N>::THREADS) col_pass_kernel(ColArgs a)
         const int b = tile / tiles_per_img, ty = tile % tiles_per_img;
         const int iy = ty * C + c;
         const size_t base = (size_t)b * N * a.ny + iy;
+        const float2 *in = a.in + (size_t)col_source(a, b) * N * a.ny + iy;
         float2 v[E];
         if (a.flags & COL_PROBE) {
             col_probe<P>(v, a, b, iy, t);
         } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = a.in[base + (size_t)(t + T * e) * a.ny];
+            for (int e = 0; e < E; ++e) v[e] = in[(size_t)(t + T * e) * a.ny];
         }
         if (a.flags & COL_FWD) fft_line<P, +1>(v, t, ad, tw);
         if (a.flags & COL_PROP) col_propagate<P>(v, a, b, iy, t);
-        if (a.flags & COL_CTF) col_ctf<P>(v, a, iy, t);
+        if (a.flags & COL_CTF) col_ctf<P>(v, a, b, iy, t);
         if (a.flags & COL_DETECT) col_detect<P, NWARP>(v, a, b, iy, t, ty, tiles_per_img, red);
         if (a.flags & COL_INV) fft_line<P, -1>(v, t, ad, tw);
         if (a.flags & COL_STORE) {
@@ -308,7 +339,7 @@ template <class PL> struct ColTmaCfg {
 
 template <class PL, int MINB>
 __global__ void __launch_bounds__(ColTmaCfg<PL>::THREADS, MINB)
-    col_tma_kernel(const __grid_constant__ CUtensorMap map, ColArgs a) {
+    col_tma_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap mapo, ColArgs a) {
     using Cfg = ColTmaCfg<PL>;
     using P = PL;
     constexpr int N = P::N;
@@ -350,7 +381,7 @@ __global__ void __launch_bounds__(ColTmaCfg<PL>::THREADS, MINB)
         mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::TILE_BYTES);
 #pragma unroll
         for (int q = 0; q < Cfg::NBOX; ++q)
-            tma_load_2d(dst + (size_t)q * Cfg::BOXR * C, &map, ty * C, b * N + q * Cfg::BOXR, &bar[s]);
+            tma_load_2d(dst + (size_t)q * Cfg::BOXR * C, &map, ty * C, col_source(a, b) * N + q * Cfg::BOXR, &bar[s]);
         issued = k + 1;
     };
     if (load && tid == 0)
@@ -390,7 +421,7 @@ __global__ void __launch_bounds__(ColTmaCfg<PL>::THREADS, MINB)
         }
         if (a.flags & COL_FWD) fft_line<P, +1>(v, t, ad, tw);
         if (a.flags & COL_PROP) col_propagate<P>(v, a, b, iy, t);
-        if (a.flags & COL_CTF) col_ctf<P>(v, a, iy, t);
+        if (a.flags & COL_CTF) col_ctf<P>(v, a, b, iy, t);
         if (a.flags & COL_DETECT) col_detect<P, Cfg::NWARP>(v, a, b, iy, t, ty, tpi, red);
         if (a.flags & COL_INV) fft_line<P, -1>(v, t, ad, tw);
         if (store) {
@@ -402,7 +433,7 @@ __global__ void __launch_bounds__(ColTmaCfg<PL>::THREADS, MINB)
             if (tid == 0) {
 #pragma unroll
                 for (int q = 0; q < Cfg::NBOX; ++q)
-                    tma_store_2d(&map, ty * C, b * N + q * Cfg::BOXR, bs + (size_t)q * Cfg::BOXR * C);
+                    tma_store_2d(&mapo, ty * C, b * N + q * Cfg::BOXR, bs + (size_t)q * Cfg::BOXR * C);
                 tma_commit();
             }
         }
@@ -572,7 +603,7 @@ __global__ void __launch_bounds__(ColHalfCfg<L>::THREADS, 1)
         fft_stage<P, 1, +1>(v, t, tw);
         const int iy = ty * C + c;
         if (a.flags & COL_PROP) col_propagate<P>(v, a, b, iy, t);
-        if (a.flags & COL_CTF) col_ctf<P>(v, a, iy, t);
+        if (a.flags & COL_CTF) col_ctf<P>(v, a, b, iy, t);
         if (a.flags & COL_DETECT) {
             float acc[kMaxDet];
 #pragma unroll
@@ -659,8 +690,8 @@ template <int N, int TH> struct RowTmaCfg {
     static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * NBUF + 1024;
 };
 
-template <int N, int TH, int MINB>
-__global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, MINB)
+template <int N, int TH, int MINB, bool IMG>
+__global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, IMG ? 1 : MINB)
     row_tma_kernel(const __grid_constant__ CUtensorMap map, RowArgs a) {
     using Cfg = RowTmaCfg<N, TH>;
     using P = Plan<N>;
@@ -672,8 +703,13 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, MINB)
     uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR);
     const int tid = threadIdx.x, t = tid % T, l = tid / T;
     const bool load = (a.flags & ROW_LOAD) != 0;
-    const int ntiles = a.nlines / L;
-    const int nmine = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int ntiles = (IMG ? a.nx : a.nlines) / L;  // of one image when they share accumulators
+    const int nmine = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * (IMG ? a.nimg : 1);
+    auto tile_of = [&](int k) {
+        if constexpr (IMG) return (int)blockIdx.x + k / a.nimg * (int)gridDim.x + k % a.nimg * ntiles;
+        else return (int)blockIdx.x + k * (int)gridDim.x;
+    };
+    [[maybe_unused]] double sum[IMG ? E : 1];
     for (int i = tid; i < TW; i += Cfg::THREADS) tw[i] = a.tw[i];
     if (tid == 0) {
         for (int s = 0; s < NBUF; ++s) mbar_init(&bar[s], 1);
@@ -683,7 +719,7 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, MINB)
     pass_begin();
     int issued = 0;
     auto issue_load = [&](int k) {
-        const int tile = blockIdx.x + k * gridDim.x, s = k % NBUF;
+        const int tile = tile_of(k), s = k % NBUF;
         fence_proxy_async();
         mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::TILE_BYTES);
         tma_load_3d(buf0 + (size_t)s * L * N, &map, 0, 0, tile * L, &bar[s]);
@@ -694,7 +730,7 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, MINB)
     int k = 0;
     bool ok = true;
     for (; k < nmine; ++k) {
-        const int tile = blockIdx.x + k * gridDim.x, s = k % NBUF;
+        const int tile = tile_of(k), s = k % NBUF;
         const int line = tile * L + l;
         float2 *bs = buf0 + (size_t)s * L * N;
         float2 *mine = bs + (size_t)l * N;
@@ -729,7 +765,9 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, MINB)
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
         }
-        if (a.flags & ROW_ACCUM) {
+        if constexpr (IMG) {
+            add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
+        } else if (a.flags & ROW_ACCUM) {
             double *acc = a.accum + (size_t)line * N;
 #pragma unroll
             for (int e = 0; e < E; ++e)
@@ -803,8 +841,8 @@ template <int N> struct RowWarpCfg {
     static_assert(P::T == 32 || P::T == 16, "warp- or half-warp-owned lines");
 };
 
-template <int N>
-__global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, RowWarpCfg<N>::MINB) row_warp_kernel(RowArgs a) {
+template <int N, bool IMG>
+__global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, IMG ? 1 : RowWarpCfg<N>::MINB) row_warp_kernel(RowArgs a) {
     using Cfg = RowWarpCfg<N>;
     using P = WarpPlan<N>;
     constexpr int E = P::E, T = P::T, LPW = Cfg::LPW, NBUF = Cfg::NBUF, W = Cfg::W, TW = plan_tw_size<P>();
@@ -834,13 +872,18 @@ __global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, RowWarpCfg<N>::MINB) r
     }
     __syncthreads();  // the only CTA barrier: tables and barriers are ready
     const bool load = (a.flags & ROW_LOAD) != 0, store = !(a.flags & ROW_NOSTORE);
-    const int nunits = a.nlines / LPW;  // units of LPW consecutive lines, one per warp at a time
+    const int nunits = (IMG ? a.nx : a.nlines) / LPW;  // units of LPW consecutive lines, one per warp at a time
     const int G = gridDim.x * W, gw = spread_id(warp, W, a.shared);
-    const int nmine = gw < nunits ? (nunits - gw + G - 1) / G : 0;
+    const int nmine = (gw < nunits ? (nunits - gw + G - 1) / G : 0) * (IMG ? a.nimg : 1);
+    auto unit_of = [&](int k) {
+        if constexpr (IMG) return gw + k / a.nimg * G + k % a.nimg * nunits;
+        else return gw + k * G;
+    };
+    [[maybe_unused]] double sum[IMG ? E : 1];
     pass_begin();
     int issued = 0;
     auto issue = [&](int k) {  // lane 0 only
-        const int unit = gw + k * G, s = k % NBUF;
+        const int unit = unit_of(k), s = k % NBUF;
         fence_proxy_async();
         mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::UNIT);
         bulk_load(ring + (size_t)s * LPW * N, a.in + (size_t)unit * LPW * N, (uint32_t)Cfg::UNIT, &bar[s]);
@@ -851,7 +894,7 @@ __global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, RowWarpCfg<N>::MINB) r
     int k = 0;
     bool ok = true;
     for (; k < nmine; ++k) {
-        const int unit = gw + k * G, s = k % NBUF, line = LPW * unit + h;
+        const int unit = unit_of(k), s = k % NBUF, line = LPW * unit + h;
         float2 *slot = ring + (size_t)s * LPW * N;
         float2 *buf = slot + (size_t)h * N;
         using Addr = typename std::conditional<Cfg::XL, RowXorLin<P>, RowXorAddr<P>>::type;
@@ -891,7 +934,9 @@ __global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, RowWarpCfg<N>::MINB) r
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
         }
-        if (a.flags & ROW_ACCUM) {
+        if constexpr (IMG) {
+            add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
+        } else if (a.flags & ROW_ACCUM) {
             double *acc = a.accum + (size_t)line * N;
 #pragma unroll
             for (int e = 0; e < E; ++e)
@@ -1055,7 +1100,109 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
     }
 }
 
-template <class P> static cudaError_t row_two_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+// Many images onto one accumulator (RowArgs::nimg) on the two-stage plans: a CTA owns
+// LPW rows of the accumulator and its four warps transform those rows of four images at
+// a time; the intensities then go through shared memory and every thread adds the four
+// images, in order, to the FP64 sums it keeps in registers.  The image order is fixed,
+// so the sums do not depend on how images are grouped into launches.  One warp walking
+// all images by itself left an SM with one warp's latencies: 165 images of 256^2 in
+// 502 us, now @RIMG@.
+template <class P>
+__global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(RowArgs a) {
+    using Cfg = RowTwoCfg<P>;
+    constexpr int N = Cfg::N, E = P::E, T = P::T, W = Cfg::W, LPW = Cfg::LPW, R0 = Cfg::R0;
+    constexpr int UNIT = LPW * N, PX = UNIT / Cfg::THREADS;
+    constexpr uint32_t AL = Cfg::ALIGN;
+    extern __shared__ unsigned char smraw[];
+    unsigned char *base = smraw + ((AL - (smem_u32(smraw) & (AL - 1u))) & (AL - 1u));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = lane / T, t = lane % T;
+    float2 *rings = reinterpret_cast<float2 *>(base), *ring = rings + (size_t)warp * 2 * UNIT;
+    float2 *tw = reinterpret_cast<float2 *>(base + Cfg::OFF_TW);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR) + warp * 2;
+    for (int i = tid; i < Cfg::TW; i += Cfg::THREADS) {
+        float sn, cn;
+        sincospif((float)(2 * (i / R0) * (i % R0)) / (float)N, &sn, &cn);  // exp(2 pi i r k / N), [r][k]
+        tw[i] = make_float2(cn, sn);
+    }
+    const float2 *twp = P::GTW ? a.tw + P::GTW_OFF : tw;
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    pass_begin();
+    const int units = a.nx / LPW, rounds = (a.nimg + W - 1) / W;
+    uint32_t issued = 0, used = 0;  // this warp's loads
+    bool ok = true;
+    int done = 0;  // units before this one
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++done) {
+        auto issue = [&](int r) {  // lane 0: this warp's image of round r, into the slot used two loads ago
+            const int img = r * W + warp;
+            if (img >= a.nimg) return;
+            const uint32_t s = issued & 1u;
+            fence_proxy_async();
+            mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::SLOT);
+            bulk_load(ring + s * UNIT, a.in + ((size_t)img * a.nx + (size_t)u * LPW) * N, (uint32_t)Cfg::SLOT, &bar[s]);
+            ++issued;
+        };
+        double *acc = a.accum + (size_t)u * UNIT;
+        double sum[PX];
+#pragma unroll
+        for (int i = 0; i < PX; ++i) sum[i] = acc[tid + Cfg::THREADS * i];
+        if (lane == 0) issue(0);
+        for (int r = 0; r < rounds; ++r) {
+            if (lane == 0 && r + 1 < rounds) issue(r + 1);
+            const bool mine = r * W + warp < a.nimg;
+            bool got = true;
+            if (mine) {
+                float2 *buf = ring + (used & 1u) * UNIT + h * N;
+                got = mbar_wait_bounded(&bar[used & 1u], (used >> 1) & 1u, kWaitLimit);
+                ++used;
+                if (!__any_sync(0xffffffffu, !got)) {
+                    float2 v[E];
+#pragma unroll
+                    for (int e = 0; e < E; ++e) v[e] = buf[t + T * e];
+                    if (a.flags & ROW_INV) {
+                        fft_line_tab<P, -1>(v, t, RowXorLin<P>{smem_u32(buf)}, twp);
+                        __syncwarp();  // every lane is done reading the slot
+#pragma unroll
+                        for (int e = 0; e < E; ++e) buf[t + T * e] = v[e];
+                    }
+                }
+            }
+            if (__syncthreads_or(!got)) {
+                ok = false;
+                break;
+            }
+            // warp q's image of this round sits in the slot of its load number
+            // done * (its images a unit) + r
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+                const int img = r * W + q;
+                if (img < a.nimg) {
+                    const double w = a.accum_wt[(a.img0 + img) % a.nw];
+                    const float2 *x = rings + ((size_t)q * 2 + ((done * ((a.nimg - q + W - 1) / W) + r) & 1)) * UNIT;
+#pragma unroll
+                    for (int i = 0; i < PX; ++i) {
+                        const float2 v = x[tid + Cfg::THREADS * i];
+                        sum[i] += w * ((double)v.x * v.x + (double)v.y * v.y);
+                    }
+                }
+            }
+            __syncthreads();  // the slots may be loaded again
+        }
+#pragma unroll
+        for (int i = 0; i < PX; ++i)
+            if (ok) acc[tid + Cfg::THREADS * i] = sum[i];
+    }
+    if (lane == 0 && !ok) {
+        if (a.err) atomicExch(a.err, 1);
+        for (uint32_t j = used; j < issued; ++j) mbar_wait_bounded(&bar[j & 1u], (j >> 1) & 1u, kWaitLimit);
+    }
+}
+
+template <class P> static cudaError_t row_two_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowTwoCfg<P>;
     static KernelSetup ks;
     int per_sm = 0;
@@ -1067,6 +1214,16 @@ template <class P> static cudaError_t row_two_launch(const RowArgs &a, cudaStrea
     int grid = nsm * per_sm < units ? nsm * per_sm : units;
     if (grid < 1) grid = 1;
     return launch_pass(row_two_kernel<P>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
+}
+template <class P> static cudaError_t row_images_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    using Cfg = RowTwoCfg<P>;
+    static KernelSetup ks;
+    int per_sm = 0;
+    cudaError_t e = ks.get(row_images_kernel<P>, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
+    if (e != cudaSuccess) return e;
+    const int units = a.nx / Cfg::LPW;
+    const int grid = nsm * per_sm < units ? nsm * per_sm : units;
+    return launch_pass(row_images_kernel<P>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
 }
 
 // ------------------------------------------ row pass, warp-pair lines, 2048
@@ -1089,7 +1246,8 @@ struct RowPairCfg {
     static_assert(HEADER < LINE && P::T == 64, "warp-pair lines");
 };
 
-__global__ void __launch_bounds__(RowPairCfg::THREADS, RowPairCfg::MINB) row_pair_kernel(RowArgs a) {
+template <bool IMG>
+__global__ void __launch_bounds__(RowPairCfg::THREADS, IMG ? 1 : RowPairCfg::MINB) row_pair_kernel(RowArgs a) {
     using Cfg = RowPairCfg;
     using P = Cfg::P;
     constexpr int N = Cfg::N, E = P::E, T = P::T, NBUF = Cfg::NBUF, PAIRS = Cfg::PAIRS;
@@ -1126,11 +1284,17 @@ __global__ void __launch_bounds__(RowPairCfg::THREADS, RowPairCfg::MINB) row_pai
     const uint32_t ring = ring0 + (uint32_t)(pr * NBUF) * LINE;
     const bool load = (a.flags & ROW_LOAD) != 0, store = !(a.flags & ROW_NOSTORE);
     const int G = gridDim.x * PAIRS, gp = spread_id(pr, PAIRS, a.shared);
-    const int nmine = gp < a.nlines ? (a.nlines - gp + G - 1) / G : 0;
+    const int rows = IMG ? a.nx : a.nlines;
+    const int nmine = (gp < rows ? (rows - gp + G - 1) / G : 0) * (IMG ? a.nimg : 1);
+    auto line_of = [&](int k) {
+        if constexpr (IMG) return gp + k / a.nimg * G + k % a.nimg * rows;
+        else return gp + k * G;
+    };
+    [[maybe_unused]] double sum[IMG ? E : 1];
     pass_begin();
     int issued = 0;
     auto issue = [&](int k) {  // the pair's first thread only
-        const int line = gp + k * G, s = k % NBUF;
+        const int line = line_of(k), s = k % NBUF;
         fence_proxy_async();
         mbar_arrive_expect_tx(&bar[s], LINE);
         bulk_load(smraw + (ring + (uint32_t)s * LINE - sbase), a.in + (size_t)line * N, LINE, &bar[s]);
@@ -1140,7 +1304,7 @@ __global__ void __launch_bounds__(RowPairCfg::THREADS, RowPairCfg::MINB) row_pai
     int k = 0;
     bool ok = true;
     for (; k < nmine; ++k) {
-        const int line = gp + k * G, s = k % NBUF;
+        const int line = line_of(k), s = k % NBUF;
         float2 *buf = reinterpret_cast<float2 *>(smraw + (ring + (uint32_t)s * LINE - sbase));
         const RowXorLin<P> ad{ring + (uint32_t)s * LINE};
         const float2 *trow = (a.flags & ROW_TRANS)
@@ -1174,7 +1338,9 @@ __global__ void __launch_bounds__(RowPairCfg::THREADS, RowPairCfg::MINB) row_pai
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
         }
-        if (a.flags & ROW_ACCUM) {
+        if constexpr (IMG) {
+            add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
+        } else if (a.flags & ROW_ACCUM) {
             double *acc = a.accum + (size_t)line * N;
 #pragma unroll
             for (int e = 0; e < E; ++e)
@@ -1202,18 +1368,18 @@ __global__ void __launch_bounds__(RowPairCfg::THREADS, RowPairCfg::MINB) row_pai
     }
 }
 
-static cudaError_t row_pair_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+template <bool IMG> static cudaError_t row_pair_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowPairCfg;
     static KernelSetup ks;
     int per_sm = 0;
     {
-        cudaError_t e = ks.get(row_pair_kernel, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
+        cudaError_t e = ks.get(row_pair_kernel<IMG>, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
         if (e != cudaSuccess) return e;
     }
-    const int units = spread_units(a.nlines, Cfg::PAIRS, a.shared);
+    const int units = spread_units(IMG ? a.nx : a.nlines, Cfg::PAIRS, a.shared);
     int grid = nsm * per_sm < units ? nsm * per_sm : units;
     if (grid < 1) grid = 1;
-    return launch_pass(row_pair_kernel, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
+    return launch_pass(row_pair_kernel<IMG>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
 }
 
 // ------------------------------------------------------------ set-up kernels
@@ -1287,7 +1453,7 @@ __global__ void detector_mask_kernel(int nx, int ny, const double *kxd, const do
 }
 
 __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
-                                 const float *ky, CtfParams p, float2 *ctf) {
+                                 const float *ky, CtfParams p, const double *df, float2 *ctf) {
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int ix = blockIdx.y;
     if (iy >= ny || ix >= nx) return;
@@ -1295,7 +1461,7 @@ __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *
     float2 out = make_float2(0.f, 0.f);
     if (k2 <= p.k2obj) {
         const double q = (double)k2;
-        double w = 0.5 * p.cs * p.lam * p.lam * q - p.df;
+        double w = 0.5 * p.cs * p.lam * p.lam * q - df[blockIdx.z];
         if (p.dfa2 != 0.0 || p.dfa3 != 0.0) {
             const double phi = atan2((double)ky[iy], (double)kx[ix]);
             w += p.dfa2 * sin(2.0 * (phi - p.dfa2phi)) +
@@ -1306,7 +1472,7 @@ __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *
         sincos(chi, &sn, &cn);
         out = make_float2((float)cn * p.scale, (float)-sn * p.scale);
     }
-    ctf[(size_t)ix * ny + iy] = out;
+    ctf[((size_t)blockIdx.z * nx + ix) * ny + iy] = out;
 }
 
 __global__ void tilt_wave_kernel(int nx, int ny, const float *xpos, const float *ypos, const float *q,
@@ -1388,19 +1554,19 @@ __global__ void detector_accumulate_kernel(int nconf, int np, int ntile, int nde
 }
 
 // ----------------------------------------------------------------- dispatch
-template <int N> static cudaError_t row_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+template <int N, bool IMG> static cudaError_t row_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     static KernelSetup ks;
     int blocks_per_sm = 0;
     {
-        cudaError_t e = ks.get(row_pass_kernel<N>, RowCfg<N>::THREADS, RowCfg<N>::SMEM, false, &blocks_per_sm);
+        cudaError_t e = ks.get(row_pass_kernel<N, IMG>, RowCfg<N>::THREADS, RowCfg<N>::SMEM, false, &blocks_per_sm);
         if (e != cudaSuccess) return e;
     }
-    const int ngroups = (a.nlines + RowCfg<N>::LPB - 1) / RowCfg<N>::LPB;
+    const int ngroups = ((IMG ? a.nx : a.nlines) + RowCfg<N>::LPB - 1) / RowCfg<N>::LPB;
     int grid = nsm * blocks_per_sm;
     if (grid > ngroups) grid = ngroups;
     if (grid < 1) grid = 1;
     dim3 block(Plan<N>::T, RowCfg<N>::LPB);
-    return launch_pass(row_pass_kernel<N>, grid, block, RowCfg<N>::SMEM, s, !a.shared, a);
+    return launch_pass(row_pass_kernel<N, IMG>, grid, block, RowCfg<N>::SMEM, s, !a.shared, a);
 }
 
 template <int N> static cudaError_t col_launch(const ColArgs &a, cudaStream_t s, int nsm) {
@@ -1453,7 +1619,7 @@ bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, con
 // aligned address; other calls take the register-only kernel.
 static bool tma_eligible(const ColArgs &a) {
     if (!a.out || ((uintptr_t)a.out & 15u)) return false;
-    if ((a.flags & COL_LOAD) && a.in != a.out) return false;
+    if ((a.flags & COL_LOAD) && a.in != a.out && (!a.fan || ((uintptr_t)a.in & 15u))) return false;
     if (!(a.flags & (COL_LOAD | COL_STORE))) return false;
     return encode_fn() != nullptr;
 }
@@ -1467,19 +1633,22 @@ template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs 
         cudaError_t e = ks.get(col_tma_kernel<PL, MINB>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
         if (e != cudaSuccess) return e;
     }
-    CUtensorMap map;
-    const cuuint64_t gdim[2] = {(cuuint64_t)a.ny, (cuuint64_t)a.batch * N};
-    const cuuint64_t gstride[1] = {(cuuint64_t)a.ny * sizeof(float2)};
-    const cuuint32_t box[2] = {(cuuint32_t)Cfg::C, (cuuint32_t)Cfg::BOXR};
-    const cuuint32_t estride[2] = {1, 1};
-    CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void *)a.out, gdim, gstride, box,
-                             estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    // waves as rows of columns; loads and stores use one map unless results fan out
+    auto encode = [&](CUtensorMap *m, const void *p, int images) {
+        const uint64_t dims[2] = {(uint64_t)a.ny, (uint64_t)images * N};
+        const uint64_t strides[1] = {(uint64_t)a.ny * sizeof(float2)};
+        const uint32_t box[2] = {(uint32_t)Cfg::C, (uint32_t)Cfg::BOXR};
+        return encode_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p, dims, strides, box,
+                                 CU_TENSOR_MAP_SWIZZLE_NONE);
+    };
+    CUtensorMap mapo, map;
+    if (!encode(&mapo, a.out, a.batch)) return cudaErrorInvalidValue;
+    map = mapo;
+    if (a.fan && !encode(&map, a.in, (a.img0 + a.batch - 1) / a.fan + 1)) return cudaErrorInvalidValue;
     const int ntiles = a.batch * (a.ny / Cfg::C);
     int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
     if (grid < 1) grid = 1;
-    return launch_pass(col_tma_kernel<PL, MINB>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, a);
+    return launch_pass(col_tma_kernel<PL, MINB>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, mapo, a);
 }
 
 template <class L> static cudaError_t col_half_launch(const ColArgs &a, cudaStream_t s, int nsm) {
@@ -1527,13 +1696,13 @@ static bool row_tma_eligible(const RowArgs &a) {
     return encode_fn() != nullptr;
 }
 
-template <int N, int TH, int MINB>
+template <int N, int TH, int MINB, bool IMG>
 static cudaError_t row_tma_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowTmaCfg<N, TH>;
     static KernelSetup ks;
     int per_sm = 0;
     {
-        cudaError_t e = ks.get(row_tma_kernel<N, TH, MINB>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
+        cudaError_t e = ks.get(row_tma_kernel<N, TH, MINB, IMG>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
         if (e != cudaSuccess) return e;
     }
     if (a.nlines % Cfg::L) return cudaErrorInvalidValue;
@@ -1546,32 +1715,33 @@ static cudaError_t row_tma_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
                              estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    const int ntiles = a.nlines / Cfg::L;
+    const int ntiles = (IMG ? a.nx : a.nlines) / Cfg::L;
     int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
     if (grid < 1) grid = 1;
-    return launch_pass(row_tma_kernel<N, TH, MINB>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, a);
+    return launch_pass(row_tma_kernel<N, TH, MINB, IMG>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, a);
 }
 
 // 128-thread CTAs, as many per SM as registers and shared memory allow (six
 // for 8-element lines): timing the 512 case, more independent CTAs beat wider
 // ones because every exchange of a line transform is a CTA-wide barrier.
 template <int N> static cudaError_t row_tma_launch(const RowArgs &a, cudaStream_t s, int nsm) {
-    return row_tma_launch_v<N, 128, (Plan<N>::E <= 8 ? 6 : 4)>(a, s, nsm);
+    constexpr int MINB = Plan<N>::E <= 8 ? 6 : 4;
+    return a.nimg ? row_tma_launch_v<N, 128, MINB, true>(a, s, nsm) : row_tma_launch_v<N, 128, MINB, false>(a, s, nsm);
 }
 
 
-template <int N> static cudaError_t row_warp_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+template <int N, bool IMG> static cudaError_t row_warp_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowWarpCfg<N>;
     static KernelSetup ks;
     int per_sm = 0;
     {
-        cudaError_t e = ks.get(row_warp_kernel<N>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
+        cudaError_t e = ks.get(row_warp_kernel<N, IMG>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
         if (e != cudaSuccess) return e;
     }
-    const int units = spread_units(a.nlines / Cfg::LPW, Cfg::W, a.shared);
+    const int units = spread_units((IMG ? a.nx : a.nlines) / Cfg::LPW, Cfg::W, a.shared);
     int grid = nsm * per_sm < units ? nsm * per_sm : units;
     if (grid < 1) grid = 1;
-    return launch_pass(row_warp_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
+    return launch_pass(row_warp_kernel<N, IMG>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
 }
 
 // Warp-owned lines for the sides whose plan fits 32 threads per line.
@@ -1814,6 +1984,19 @@ static TcPassArgs tc_col_args(int nx, const ColArgs &a) {
     return t;
 }
 
+template <class P> static cudaError_t row_two_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    return a.nimg ? row_images_launch<P>(a, s, nsm) : row_two_launch_v<P>(a, s, nsm);
+}
+template <int N> static cudaError_t row_warp_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    return a.nimg ? row_warp_launch_v<N, true>(a, s, nsm) : row_warp_launch_v<N, false>(a, s, nsm);
+}
+static cudaError_t row_pair_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    return a.nimg ? row_pair_launch_v<true>(a, s, nsm) : row_pair_launch_v<false>(a, s, nsm);
+}
+template <int N> static cudaError_t row_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    return a.nimg ? row_launch_v<N, true>(a, s, nsm) : row_launch_v<N, false>(a, s, nsm);
+}
+
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches) {
     const int fam0 = sched_row(ny);
     if (fam0 == FAM_TC && row_tc_eligible(ny, a)) return launch_tc_pass(tc_row_args(ny, a), s, nsm, launches);
@@ -1920,11 +2103,11 @@ cudaError_t launch_detector_mask(int nx, int ny, const double *kxd, const double
 }
 
 cudaError_t launch_ctf_table(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
-                             const float *ky, const CtfParams &p, float2 *ctf, cudaStream_t s,
-                             int64_t *launches) {
+                             const float *ky, const CtfParams &p, const double *df, int ndf, float2 *ctf,
+                             cudaStream_t s, int64_t *launches) {
     ++*launches;
-    dim3 grid((ny + 255) / 256, nx);
-    ctf_table_kernel<<<grid, 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, ctf);
+    dim3 grid((ny + 255) / 256, nx, ndf);
+    ctf_table_kernel<<<grid, 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, df, ctf);
     return cudaGetLastError();
 }
 

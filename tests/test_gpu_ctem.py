@@ -190,3 +190,44 @@ def test_ctem_image_vs_compiled_reference(ctx, golden, ci):
     img, _, _ = ctx.ctem_image(S["t"], dz, S["seq"], ax, by, kev, L["cs"], L["df"], L["k_obj"],
                                df_spread=L["df_spread"], df_step=L["df_step"], astig=L["astig"])
     assert O.rel_l2(img, G[f"pc_{ci}_pix"]) < 2e-5
+
+
+# every row kernel that sums images (TMA tiles, two-stage lines, warp lines, warp pairs,
+# registers only), image counts that leave the last round of four uneven
+@pytest.mark.parametrize("nx,ny,family", [(64, 64, 0), (64, 128, 0), (128, 256, 0), (64, 384, 0), (64, 512, 0),
+                                          (64, 768, 0), (64, 1024, 0), (64, 2048, 0), (128, 256, 1), (64, 256, 2),
+                                          (64, 64, 2)])
+def test_many_images_onto_one_accumulator_vs_oracle(nx, ny, family):
+    from multislice_gb300 import Context
+    rng = np.random.default_rng(nx + ny)
+    ax, by, kev, dz = 11.0, 11.0 * ny / nx, 200.0, 1.7
+    V = np.zeros((2, nx, ny))
+    for l in range(2):
+        V[l, rng.integers(0, nx, 20), rng.integers(0, ny, 20)] = rng.uniform(50, 400, 20)
+    t = O.transmission(V, kev, ax, by, np.complex64)
+    seq = [0, 1, 0]
+    props = [O.propagator_tables(nx, ny, ax, by, kev, dz, precision="f64")] * 2
+    mask = O.band_mask(nx, ny, ax, by)
+    with Context(0) as c:
+        for n in {nx, ny}:
+            old = c.get_schedule(n)
+            c.set_schedule(n, family, family)
+        try:
+            img, na = c.partial_coherence(t, dz, seq, ax, by, kev, CS, DF, 1.5, 0.0, 2.4e-3, df_spread=30.0,
+                                          df_step=20.0)
+            psi = np.ones((3, nx, ny), np.complex64)
+            exi = np.zeros((nx, ny))
+            img2, w, _ = c.ctem_image(t, dz, seq, ax, by, kev, CS, DF, 1.5, psi=psi, df_spread=30.0, df_step=20.0,
+                                      exit_intensity=exi)
+        finally:
+            for n in {nx, ny}:
+                c.set_schedule(n, 0, 0)
+    assert old == (0, 0)
+    ref, nref = O.partial_coherence(t.astype(np.complex128), props, seq, mask, ax, by, kev, CS, DF, 1.5, 0.0, 2.4e-3,
+                                    30.0, 20.0)
+    assert na == nref and na > 1
+    assert O.rel_l2(img, ref) < 2e-5
+    w0, _ = O.multislice(np.ones((nx, ny), np.complex128), t.astype(np.complex128), props, seq, mask)
+    assert O.rel_l2(w[2], w0) < 2e-5
+    assert O.rel_l2(exi, 3 * np.abs(w0) ** 2) < 2e-5
+    assert O.rel_l2(img2, 3 * O.ctem_image(w0, ax, by, kev, CS, DF, 1.5, 30.0, 20.0)) < 2e-5
