@@ -550,7 +550,7 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     // The spectra W = Psi(k) / (nx ny) of the batch fan out to batch x ndf images, a
     // chunk at a time: one column pass (times the table, inverse) into the chunk's
     // buffer, one row pass that adds the images in order.  One image at a time cost
-    // three launches each (15 angles x 11 defocus values at 256^2: 1.6 ms, now @IMG@).
+    // three launches each (15 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
     const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
     // A context with a memory cap keeps to one image's buffer.
     size_t chunk = c->mem.limit ? 1 : std::max<size_t>(1, std::min(total, ((size_t)512 << 20) / ibytes));
