@@ -941,21 +941,18 @@ namespace {
 
 // Host half of a potential build: the atoms validated and binned by slice
 // (stably, so the sum order inside a slice is the input order), the
-// per-species parameters and radial tables, laid out as one upload image
-// off | ic | jc | fx | fy | Z | sp | xf | yf | tab | zslot.  Each atom is
-// given as its nearest pixel (ic, jc) and the residue x - ic dxp, y - jc dyp
-// formed in FP64 and rounded to float.  The radial tables are kept and reused
-// while the species, the cutoff and the FPARAMS table stay the same.
+// per-species parameters, laid out as one upload image
+// off | ic | jc | fx | fy | Z | sp | xf | yf | rows | zslot; the device appends the
+// radial tables made from the species' FPARAMS rows.  Each atom is given as its
+// nearest pixel (ic, jc) and the residue x - ic dxp, y - jc dyp formed in FP64 and
+// rounded to float.
 struct PotImage {
     std::vector<unsigned char> h;
-    size_t o_off = 0, o_ic = 0, o_jc = 0, o_fx = 0, o_fy = 0, o_z = 0, o_sp = 0, o_xf = 0, o_yf = 0, o_tab = 0,
+    size_t o_off = 0, o_ic = 0, o_jc = 0, o_fx = 0, o_fy = 0, o_z = 0, o_sp = 0, o_xf = 0, o_yf = 0, o_rows = 0, o_tab = 0,
            o_zs = 0;
+    size_t bytes = 0;  // with the tables, after h
     int nsp = 0;
     double tab_r0 = 0.15;
-    std::vector<int> tab_z;
-    double tab_radius = -1.0;
-    const double *tab_fp = nullptr;
-    std::vector<float4> tab;
 };
 
 int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, const msl_grid *g, int nslice,
@@ -969,6 +966,7 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
         return fail(c, MSL_E_ARG, "atom arrays are required");
     const double dz = at->cz / nslice;
     std::vector<int> kz(at->natom), count(nslice + 1, 0);
+    bool used[104] = {false};
     for (int i = 0; i < at->natom; ++i) {
         if (!is_fin(at->x[i]) || !is_fin(at->y[i]) || !is_fin(at->z[i]))
             return fail(c, MSL_E_ARG, "atom coordinates must be finite (atom " + std::to_string(i) + ")");
@@ -977,16 +975,16 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
         if (k >= 0 && (at->Z[i] < 1 || at->Z[i] > 103))
             return fail(c, MSL_E_ARG, "atomic number out of range 1..103 (atom " + std::to_string(i) + ")");
         kz[i] = k;
-        if (k >= 0) count[k + 1]++;
+        if (k >= 0) {
+            count[k + 1]++;
+            used[at->Z[i]] = true;
+        }
     }
     for (int k = 0; k < nslice; ++k) count[k + 1] += count[k];
     const int nkeep = count[nslice];
     const size_t nk = nkeep > 0 ? (size_t)nkeep : 1;
     // per-species float parameters: A = AL a, B = 2 pi sqrt(b), C = AG c / d, D = pi^2 / d
     // (constants of slicelib.cpp:2673-2674)
-    bool used[104] = {false};
-    for (int i = 0; i < at->natom; ++i)
-        if (kz[i] >= 0) used[at->Z[i]] = true;
     const double AL = 300.8242834, AG = 150.4121417, PIK = 3.141592654;
     std::vector<float> sp(104 * 12, 0.f);
     for (int z = 1; z <= 103; ++z) {
@@ -1002,8 +1000,8 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
             sp[z * 12 + 7 + 2 * i] = (float)(PIK * PIK / d);
         }
     }
-    // tabulated radial profiles of the species present (up to kPotMaxSp): cubic
-    // pieces of vzatom evaluated in FP64 over [0.15 A, radius]
+    // species present (up to kPotMaxSp of them take tabulated radial profiles: cubic
+    // pieces of vzatom evaluated in FP64 over [0.15 A, radius])
     std::vector<int> zlist, zslot(104, -1);
     for (int z = 1; z <= 103; ++z)
         if (used[z]) {
@@ -1011,14 +1009,6 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
             zlist.push_back(z);
         }
     im.nsp = (zlist.size() <= (size_t)msl::kPotMaxSp && radius > 2 * im.tab_r0) ? (int)zlist.size() : 0;
-    const size_t ntab = (size_t)std::max(im.nsp, 1) * msl::kPotTabN;
-    if (im.tab_z != zlist || im.tab_radius != radius || im.tab_fp != fparams || im.tab.size() != ntab) {
-        im.tab.assign(ntab, make_float4(0.f, 0.f, 0.f, 0.f));
-        if (im.nsp) msl::potential_tables(fparams, zlist.data(), im.nsp, im.tab_r0, radius, im.tab.data());
-        im.tab_z = zlist;
-        im.tab_radius = radius;
-        im.tab_fp = fparams;
-    }
     auto up16 = [](size_t x) { return ((x + 15) / 16) * 16; };
     im.o_off = 0;
     im.o_ic = up16(sizeof(int) * (nslice + 1));
@@ -1029,9 +1019,11 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
     im.o_sp = up16(im.o_z + sizeof(int) * nk);
     im.o_xf = up16(im.o_sp + sizeof(float) * sp.size());
     im.o_yf = up16(im.o_xf + sizeof(float) * nk);
-    im.o_tab = up16(im.o_yf + sizeof(float) * nk);
-    im.o_zs = im.o_tab + sizeof(float4) * im.tab.size();
-    im.h.assign(im.o_zs + sizeof(int) * zslot.size(), 0);
+    im.o_rows = up16(im.o_yf + sizeof(float) * nk);
+    im.o_zs = im.o_rows + sizeof(double) * 12 * im.nsp;
+    im.o_tab = up16(im.o_zs + sizeof(int) * zslot.size());
+    im.h.assign(im.o_tab, 0);
+    im.bytes = im.o_tab + sizeof(float4) * im.nsp * msl::kPotTabN;
     unsigned char *h = im.h.data();
     int *ics = (int *)(h + im.o_ic), *jcs = (int *)(h + im.o_jc), *zs = (int *)(h + im.o_z);
     float *fxs = (float *)(h + im.o_fx), *fys = (float *)(h + im.o_fy);
@@ -1056,14 +1048,23 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
     }
     memcpy(h + im.o_off, count.data(), sizeof(int) * (nslice + 1));
     memcpy(h + im.o_sp, sp.data(), sizeof(float) * sp.size());
-    memcpy(h + im.o_tab, im.tab.data(), sizeof(float4) * im.tab.size());
+    for (int i = 0; i < im.nsp; ++i)
+        memcpy(h + im.o_rows + sizeof(double) * 12 * i, fparams + zlist[i] * 12, sizeof(double) * 12);
     memcpy(h + im.o_zs, zslot.data(), sizeof(int) * zslot.size());
     return MSL_OK;
 }
 
-// Device half: launch the gather on the upload image at `d` (device memory).
-int potential_launch(msl_ctx *c, const PotImage &im, const unsigned char *d, const msl_grid *g, int nslice,
+// Device half: the radial tables, then the gather, on the upload image at `d` (device
+// memory of im.bytes).
+int potential_launch(msl_ctx *c, const PotImage &im, unsigned char *d, const msl_grid *g, int nslice,
                      double radius, float *vd) {
+    // the table reaches 2e-6 beyond the cutoff, so no pixel inside rounds past its end
+    const double h = (radius * (1.0 + 2e-6) - im.tab_r0) / msl::kPotTabN;
+    if (im.nsp)
+        LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] {
+                       return msl::launch_potential_tables((const double *)(d + im.o_rows), im.nsp, im.tab_r0, h,
+                                                           (float4 *)(d + im.o_tab), c->stream, &c->launches);
+                   }));
     msl::PotArgs a;
     a.ic = (const int *)(d + im.o_ic);
     a.jc = (const int *)(d + im.o_jc);
@@ -1088,9 +1089,8 @@ int potential_launch(msl_ctx *c, const PotImage &im, const unsigned char *d, con
     a.tab = (const float4 *)(d + im.o_tab);
     a.zslot = (const int *)(d + im.o_zs);
     a.nsp = im.nsp;
-    a.tab_r0 = (float)im.tab_r0;
-    a.tab_inv_h = (float)(msl::kPotTabN / (radius - im.tab_r0));
-    a.tab_off = (float)(-im.tab_r0 * msl::kPotTabN / (radius - im.tab_r0));
+    a.tab_inv_h = (float)(1.0 / h);
+    a.tab_off = (float)(-im.tab_r0 / h - 0.5);
     LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] { return msl::launch_potential(a, c->stream, &c->launches); }));
     return MSL_OK;
 }
@@ -1204,7 +1204,7 @@ struct PhononBuilder {
         const int sl = cfg & 1;
         if (prepared[sl] != cfg && (rc = prepare(cfg))) return rc;
         const PotImage &m = im[sl];
-        const size_t bytes = m.h.size();
+        const size_t bytes = m.h.size(), dbytes = m.bytes;
         if (bytes > pin_cap) {  // (re)allocate both pinned buffers with headroom
             for (int i = 0; i < 2; ++i) {
                 CUDA_TRY(c, cudaEventSynchronize(ev[i]));
@@ -1214,15 +1214,15 @@ struct PhononBuilder {
             pin_cap = bytes + bytes / 4;
             for (int i = 0; i < 2; ++i) CUDA_TRY(c, cudaHostAlloc((void **)&pin[i], pin_cap, cudaHostAllocDefault));
         }
-        if (bytes > atoms.cap) {  // growth frees the old buffer: let the stream drain first
+        if (dbytes > atoms.cap) {  // growth frees the old buffer: let the stream drain first
             CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-            CUDA_TRY(c, atoms.ensure(bytes + bytes / 4));
+            CUDA_TRY(c, atoms.ensure(dbytes + dbytes / 4));
         }
         CUDA_TRY(c, cudaEventSynchronize(ev[sl]));  // the upload two configurations back has read pin[sl]
         memcpy(pin[sl], m.h.data(), bytes);
         CUDA_TRY(c, cudaMemcpyAsync(atoms.p, pin[sl], bytes, cudaMemcpyHostToDevice, c->stream));
         CUDA_TRY(c, cudaEventRecord(ev[sl], c->stream));
-        if ((rc = potential_launch(c, m, (const unsigned char *)atoms.p, g, nslice, radius, (float *)pot.p))) return rc;
+        if ((rc = potential_launch(c, m, (unsigned char *)atoms.p, g, nslice, radius, (float *)pot.p))) return rc;
         if ((rc = transmission_enqueue(c, g, o, (const float *)pot.p, nslice, t, st, twr, twc))) return rc;
         if (cfg + 1 < nconfig && (rc = prepare(cfg + 1))) return rc;
         return MSL_OK;
@@ -1880,6 +1880,7 @@ int msl_potential_build(msl_ctx *c, const msl_atoms *at, const double *fparams, 
     PotImage im;
     if ((rc = potential_prepare(c, at, fparams, g, nslice, radius, im))) return rc;
     CUDA_TRY(c, cudaSetDevice(c->device));
+    CUDA_TRY(c, c->atoms.ensure(im.bytes));
     if ((rc = upload(c, c->atoms, im.h.data(), im.h.size()))) return rc;
     const size_t vbytes = sizeof(float) * (size_t)nslice * g->nx * g->ny;
     float *vd;
@@ -1890,7 +1891,7 @@ int msl_potential_build(msl_ctx *c, const msl_atoms *at, const double *fparams, 
         CUDA_TRY(c, c->pot.ensure(vbytes));
         vd = (float *)c->pot.p;
     }
-    if ((rc = potential_launch(c, im, (const unsigned char *)c->atoms.p, g, nslice, radius, vd))) return rc;
+    if ((rc = potential_launch(c, im, (unsigned char *)c->atoms.p, g, nslice, radius, vd))) return rc;
     if (!vdev) CUDA_TRY(c, cudaMemcpyAsync(v_out, vd, vbytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     collect_profile(c);

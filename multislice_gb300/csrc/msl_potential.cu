@@ -26,7 +26,14 @@
 // columns and 32 rows are formed once per tile and the pair loop runs in FP32
 // on them.  Every pixel sums its atoms in atom order, whatever the tile shape.
 // 64-pixel-wide tiles halve the per-pixel share of the per-atom work against
-// 32 x 32 (Au 2048^2: 2.78 ms per configuration against 3.40).
+// 32 x 32 (Au 2048^2: 2.78 ms per configuration against 3.40).  A warp's pixels are
+// blocks of 4 x 8, so that a block is mostly all inside or all outside a cutoff and its
+// lanes look up neighbouring table pieces; the piece number comes from a float
+// addition, not conversions (a quarter-rate pipe).  What bounds it: the
+// 16-byte table gathers (shared-memory wavefronts at 78 % of peak) and issue (76 %):
+// SrTiO3, 100 slices of 512^2, 5 A cutoff: 0.50 ms (0.69 with warps of 32 rows x 1
+// column, converted piece numbers and a branch per pixel); Au 2048^2, 40 slices, 3 A:
+// 1.10 ms (1.42).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -39,6 +46,7 @@ namespace {
 // tile shape and list capacity picked by timing 16 / 32 / 64 / 128-pixel-wide tiles
 // and 32 / 64 / 128-atom lists on the Au 2048^2 potentials
 constexpr int TX = 64, TY = 32, THREADS = 256, PX = TX * TY / THREADS, CAP = 64;
+static_assert(TX == 64 && TY == 32 && THREADS == 256 && PX == 8, "a warp covers 32 x 8 pixels in blocks of 4 x 8");
 constexpr int KR = 2, ROUND = KR * THREADS, NW = THREADS / 32;  // atoms culled per thread per round
 
 __device__ __forceinline__ float poly(const float *c, int n, float t) {
@@ -53,6 +61,14 @@ __constant__ float kK0A[7] = {-0.57721566f, 0.42278420f, 0.23069756f, 0.03488590
 __constant__ float kK0B[7] = {1.25331414f, -0.07832358f, 0.02189568f, -0.01062446f, 0.00587872f,
                               -0.00251540f, 0.00053208f};
 
+constexpr float kRound = 12582912.0f;  // 1.5 2^23: adding it rounds to an integer
+// 1 / sqrt(x) of x > 0, denormals taken as 0.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // K0(x), x > 0 (A&S 9.8.5 for x <= 2 with I0 from 9.8.1, 9.8.6 above).
 __device__ __forceinline__ float bessk0f(float x) {
     if (x <= 2.0f) {
@@ -63,6 +79,16 @@ __device__ __forceinline__ float bessk0f(float x) {
     }
     return expf(-x) * poly(kK0B, 7, 2.0f / x) * rsqrtf(x);
 }
+// vzatom at r = max(sqrt(r2), 1e-10 A); p: A1 B1 A2 B2 A3 B3 C1 D1 C2 D2 C3 D3
+__device__ __noinline__ float pot_analytic(const float *p, float r2) {
+    const float r = sqrtf(fmaxf(r2, 1.0e-20f));
+    float v = __ldg(p + 0) * bessk0f(__ldg(p + 1) * r) + __ldg(p + 2) * bessk0f(__ldg(p + 3) * r) +
+              __ldg(p + 4) * bessk0f(__ldg(p + 5) * r);
+    const float rr = r * r;
+    v += __ldg(p + 6) * expf(-__ldg(p + 7) * rr) + __ldg(p + 8) * expf(-__ldg(p + 9) * rr) +
+         __ldg(p + 10) * expf(-__ldg(p + 11) * rr);
+    return v;
+}
 }  // namespace
 
 template <bool TAB>
@@ -72,22 +98,24 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
     __shared__ int sS[CAP];
     __shared__ int sic[CAP], sjc[CAP];
     __shared__ float sfx[CAP], sfy[CAP];
-    __shared__ float sdx[CAP][TX];
+    __shared__ __align__(16) float sdx[CAP][TX];  // [half][lane column][block]: a thread's eight in a row
     __shared__ float sdy[CAP][TY];
     __shared__ int wcount[KR * NW];
     const int tid = threadIdx.x;
     if (TAB) {
         for (int i = tid; i < a.nsp * kPotTabN; i += THREADS) stab[i] = a.tab[i];
     }
-    const int ty = tid % TY, txg = tid / TY;  // pixels (txg + 8 j, ty), j < PX
     const int lane = tid & 31, warp = tid >> 5;
+    // a warp's pixel block j: 4 columns (along x) of 8 neighbouring rows (along y)
+    const int ty = 8 * (warp & 3) + (lane & 7), tx = 32 * (warp >> 2) + (lane >> 3);  // pixels (tx + 4 j, ty), j < PX
+    const int txs = 8 * (4 * (warp >> 2) + (lane >> 3));
     const int iy0 = blockIdx.x * TY, ix0 = blockIdx.y * TX, s = blockIdx.z;
 
     // tile bounding box (pixel positions) for the culling, in float with a margin
     // that covers the float rounding of the coordinates (the culling only has to
     // keep every atom that can reach the tile; the pair loop tests r < radius)
-    const float xc = (float)((ix0 + 0.5 * (TX - 1)) * a.dxp), hx = (float)(0.5 * (TX - 1) * a.dxp);
-    const float yc = (float)((iy0 + 0.5 * (TY - 1)) * a.dyp), hy = (float)(0.5 * (TY - 1) * a.dyp);
+    const float xc = ((float)ix0 + 0.5f * (TX - 1)) * a.dxpf, hx = 0.5f * (TX - 1) * a.dxpf;
+    const float yc = ((float)iy0 + 0.5f * (TY - 1)) * a.dypf, hy = 0.5f * (TY - 1) * a.dypf;
     const float axf = (float)a.ax, byf = (float)a.by;
     const float rad = sqrtf(a.rad2) * (1.0f + 1e-5f) + 1e-3f;
     const int a0 = a.off[s], a1 = a.off[s + 1];
@@ -166,7 +194,7 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
                 int m = sic[k] - (ix0 + i);
                 if (2 * m >= a.nx) m -= a.nx;
                 else if (2 * m < -a.nx) m += a.nx;
-                sdx[k][i] = fabsf(fmaf((float)m, a.dxpf, sfx[k]));
+                sdx[k][8 * (4 * (i >> 5) + (i & 3)) + ((i >> 2) & 7)] = fabsf(fmaf((float)m, a.dxpf, sfx[k]));
             }
             for (int idx = tid; idx < n * TY; idx += THREADS) {
                 const int k = idx / TY, i = idx % TY;
@@ -177,44 +205,34 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
             }
             __syncthreads();
             for (int k = 0; k < n; ++k) {
-                // a warp holds 32 rows x 4 columns of the tile (ty = lane, the
-                // columns txg + 8 j warp-uniform): an atom whose x offset puts all
-                // four columns beyond the cutoff is skipped by the whole warp
-                float dx[PX];
-#pragma unroll
-                for (int j = 0; j < PX; ++j) dx[j] = sdx[k][txg + 8 * j];
-                float dxm = dx[0];
-#pragma unroll
-                for (int j = 1; j < PX; ++j) dxm = fminf(dxm, dx[j]);
-                if (dxm * dxm >= a.rad2) continue;
+                // the warp stays together: a block with no pixel inside the cutoff is skipped,
+                // in any other every lane goes through the table and the outer ones drop it
                 const float dy = sdy[k][ty], dy2 = dy * dy;
-                if (dy2 >= a.rad2) continue;
-                const float *p = a.sp + sZ[k] * 12;
+                if (!__any_sync(0xffffffffu, dy2 < a.rad2)) continue;
+                const float4 d0 = *(const float4 *)&sdx[k][txs], d1 = *(const float4 *)&sdx[k][txs + 4];
+                const float dx[PX] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
                 const float4 *tb = TAB ? stab + sS[k] * kPotTabN : nullptr;
 #pragma unroll
                 for (int j = 0; j < PX; ++j) {
                     const float r2 = fmaf(dx[j], dx[j], dy2);
-                    if (r2 < a.rad2) {
-                        // r = max(r, 1e-10 A) through the reciprocal square root
-                        const float r2c = fmaxf(r2, 1.0e-20f);
-                        const float r = r2c * rsqrtf(r2c);
-                        if (TAB && r >= a.tab_r0) {
-                            // cubic piece of the tabulated profile: ((c3 t + c2) t + c1) t + c0
-                            const float u = fmaf(r, a.tab_inv_h, a.tab_off);
-                            const int i = min((int)u, kPotTabN - 1);
-                            const float t = u - (float)i;
-                            const float4 c = tb[i];
-                            acc[j] += fmaf(fmaf(fmaf(c.w, t, c.z), t, c.y), t, c.x);
-                            continue;
-                        }
-                        float v = __ldg(p + 0) * bessk0f(__ldg(p + 1) * r) +
-                                  __ldg(p + 2) * bessk0f(__ldg(p + 3) * r) +
-                                  __ldg(p + 4) * bessk0f(__ldg(p + 5) * r);
-                        const float rr = r * r;
-                        v += __ldg(p + 6) * expf(-__ldg(p + 7) * rr) + __ldg(p + 8) * expf(-__ldg(p + 9) * rr) +
-                             __ldg(p + 10) * expf(-__ldg(p + 11) * rr);
-                        acc[j] += v;
+                    const bool in = r2 < a.rad2;
+                    if (!__any_sync(0xffffffffu, in)) continue;
+                    float v = 0.f;
+                    bool near = true;  // below the table: the analytic form
+                    if (TAB) {
+                        // cubic piece of the tabulated profile in t = u - i, |t| <= 1/2, about the
+                        // middle of the piece i nearest u: rounded by adding 1.5 2^23, so that no
+                        // pair takes a conversion (a pixel beyond the cutoff lands on any piece;
+                        // r = 0 gives a NaN and takes the analytic form)
+                        const float u = fmaf(r2 * rsqrt_normal(r2), a.tab_inv_h, a.tab_off);
+                        const float m = u + kRound;
+                        const float t = u - (m - kRound);
+                        const float4 c = tb[__float_as_int(m) & (kPotTabN - 1)];
+                        v = fmaf(fmaf(fmaf(c.w, t, c.z), t, c.y), t, c.x);
+                        near = !(u >= -0.5f);
                     }
+                    if (near && in) v = pot_analytic(a.sp + sZ[k] * 12, r2);
+                    if (in) acc[j] += v;
                 }
             }
         }
@@ -222,7 +240,7 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
     const int iy = iy0 + ty;
 #pragma unroll
     for (int j = 0; j < PX; ++j) {
-        const int ix = ix0 + txg + 8 * j;
+        const int ix = ix0 + tx + 4 * j;
         if (ix < a.nx && iy < a.ny) a.v[((size_t)s * a.nx + ix) * a.ny + iy] = acc[j];
     }
 }
@@ -244,30 +262,28 @@ cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches
 }
 
 // ------------------------------------------------------------ radial tables
+// Cubic pieces of vzatom evaluated in FP64 (slicelib.cpp:2666-2716 with the A&S Bessel
+// polynomials of :168-235), kPotTabN of width h from r0 per species: the cubic through
+// the profile at t = -1/2, -1/6, 1/6, 1/2 about the middle of piece i, a thread per
+// point.  On one host core the three species of SrTiO3 took 218 us a call.
 namespace {
-// vzatom in double (slicelib.cpp:2666-2716 with the A&S Bessel polynomials of :168-235)
-double bessi0d(double x) {
-    static const double c[7] = {1.0, 3.5156229, 3.0899424, 1.2067492, 0.2659732, 0.0360768, 0.0045813};
-    const double t = (x / 3.75) * (x / 3.75);
+__device__ __forceinline__ double polyd(const double *c, double t) {
     double s = c[6];
+#pragma unroll
     for (int i = 5; i >= 0; --i) s = s * t + c[i];
     return s;
 }
-double bessk0d(double x) {
-    static const double a[7] = {-0.57721566, 0.42278420, 0.23069756, 0.03488590, 0.00262698, 0.00010750, 0.00000740};
-    static const double b[7] = {1.25331414, -0.07832358, 0.02189568, -0.01062446, 0.00587872, -0.00251540, 0.00053208};
+__constant__ double kI0D[7] = {1.0, 3.5156229, 3.0899424, 1.2067492, 0.2659732, 0.0360768, 0.0045813};
+__constant__ double kK0AD[7] = {-0.57721566, 0.42278420, 0.23069756, 0.03488590, 0.00262698, 0.00010750, 0.00000740};
+__constant__ double kK0BD[7] = {1.25331414, -0.07832358, 0.02189568, -0.01062446, 0.00587872, -0.00251540, 0.00053208};
+__device__ double bessk0d(double x) {
     if (x <= 2.0) {
-        const double t = 0.25 * x * x;
-        double s = a[6];
-        for (int i = 5; i >= 0; --i) s = s * t + a[i];
-        return -log(0.5 * x) * bessi0d(x) + s;
+        const double q = (x / 3.75) * (x / 3.75);
+        return -log(0.5 * x) * polyd(kI0D, q) + polyd(kK0AD, 0.25 * x * x);
     }
-    const double t = 2.0 / x;
-    double s = b[6];
-    for (int i = 5; i >= 0; --i) s = s * t + b[i];
-    return exp(-x) * s / sqrt(x);
+    return exp(-x) * polyd(kK0BD, 2.0 / x) / sqrt(x);
 }
-double vz_double(const double *f, double r) {
+__device__ double vz_double(const double *f, double r) {
     const double AL = 300.8242834, AG = 150.4121417, PIK = 3.141592654;
     const double x = 2.0 * PIK * r;
     double suml = 0.0, sumg = 0.0;
@@ -276,24 +292,32 @@ double vz_double(const double *f, double r) {
     for (int i = 0; i < 3; ++i) sumg += f[6 + 2 * i] * exp(-x2 / f[7 + 2 * i]) / f[7 + 2 * i];
     return AL * suml + AG * sumg;
 }
+constexpr int TAB_THREADS = 64;
+__global__ void __launch_bounds__(TAB_THREADS)
+    potential_tables_kernel(const double *rows, double r0, double h, float4 *out) {
+    // four neighbouring lanes hold a piece's four points
+    const int piece = (blockIdx.x * TAB_THREADS + threadIdx.x) >> 2, q = threadIdx.x & 3;
+    const double r = r0 + piece * h;
+    const double y = vz_double(rows + blockIdx.y * 12, q == 0 ? r : q == 1 ? r + h / 3 : q == 2 ? r + 2 * h / 3 : r + h);
+    const int l0 = threadIdx.x & 28;
+    const double y0 = __shfl_sync(0xffffffffu, y, l0), y1 = __shfl_sync(0xffffffffu, y, l0 + 1),
+                 y2 = __shfl_sync(0xffffffffu, y, l0 + 2), y3 = __shfl_sync(0xffffffffu, y, l0 + 3);
+    if (q == 0) {
+        const double s0 = y1 + y2, s1 = y0 + y3, d0 = y2 - y1, d1 = y3 - y0;
+        out[blockIdx.y * kPotTabN + piece] =
+            make_float4((float)((9 * s0 - s1) / 16), (float)((27 * d0 - d1) / 8), (float)(9 * (s1 - s0) / 4),
+                        (float)(9 * (d1 - 3 * d0) / 2));
+    }
+}
 }  // namespace
 
-void potential_tables(const double *fparams, const int *zlist, int nsp, double r0, double rmax, float4 *out) {
-    const double h = (rmax - r0) / kPotTabN;
-    for (int sidx = 0; sidx < nsp; ++sidx) {
-        const double *f = fparams + zlist[sidx] * 12;
-        for (int i = 0; i < kPotTabN; ++i) {
-            // the cubic through the profile at t = 0, 1/3, 2/3, 1 of [r0 + i h, r0 + (i + 1) h]
-            const double r = r0 + i * h;
-            const double y0 = vz_double(f, r), y1 = vz_double(f, r + h / 3), y2 = vz_double(f, r + 2 * h / 3),
-                         y3 = vz_double(f, r + h);
-            const double c0 = y0;
-            const double c1 = (-11 * y0 + 18 * y1 - 9 * y2 + 2 * y3) / 2;
-            const double c2 = 9 * (2 * y0 - 5 * y1 + 4 * y2 - y3) / 2;
-            const double c3 = 27 * (-y0 + 3 * y1 - 3 * y2 + y3) / 6;
-            out[(size_t)sidx * kPotTabN + i] = make_float4((float)c0, (float)c1, (float)c2, (float)c3);
-        }
-    }
+cudaError_t launch_potential_tables(const double *rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,
+                                    int64_t *launches) {
+    ++*launches;
+    static_assert(4 * kPotTabN % TAB_THREADS == 0, "whole blocks of pieces");
+    potential_tables_kernel<<<dim3(4 * kPotTabN / TAB_THREADS, nsp), TAB_THREADS, 0, s>>>(
+        rows, r0, h, out);
+    return cudaGetLastError();
 }
 
 }  // namespace msl
