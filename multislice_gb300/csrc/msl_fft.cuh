@@ -326,12 +326,31 @@ template <int DIR, bool PK> __device__ __forceinline__ void dft12(float2 *a) {
     }
 }
 
+// 24 = 3 x 8 coprime (Good-Thomas): inputs 3 n1 + 8 n2, outputs 9 k1 + 16 k2 (mod 24),
+// no twiddles between the factors.
+template <int DIR, bool PK> __device__ __forceinline__ void dft24(float2 *a) {
+    float2 x[3][8];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < 8; ++n1) x[n2][n1] = a[(3 * n1 + 8 * n2) % 24];
+        dft8<DIR, PK>(x[n2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 8; ++k1) {
+        dft3<DIR, PK>(x[0][k1], x[1][k1], x[2][k1]);
+#pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) a[(9 * k1 + 16 * k2) % 24] = x[k2][k1];
+    }
+}
+
 template <int R, int DIR, bool PK> __device__ __forceinline__ void dft(float2 *a) {
     if constexpr (R == 2) dft2<DIR, PK>(a[0], a[1]);
     else if constexpr (R == 3) dft3<DIR, PK>(a[0], a[1], a[2]);
     else if constexpr (R == 4) dft4<DIR, PK>(a[0], a[1], a[2], a[3]);
     else if constexpr (R == 6) dft6<DIR, PK>(a);
     else if constexpr (R == 12) dft12<DIR, PK>(a);
+    else if constexpr (R == 24) dft24<DIR, PK>(a);
     else if constexpr (R == 8) dft8<DIR, PK>(a);
     else if constexpr (R == 16) dft16<DIR, PK>(a);
     else if constexpr (R == 32) dft32<DIR, PK>(a);
@@ -742,32 +761,81 @@ __device__ __forceinline__ void fft_line_tab(float2 (&v)[P::E], int t, const Row
     }
 }
 
-// Plan with one warp per line (same radices as Plan<N>).  OWN_TW: the kernel
-// builds its twiddle tables (radices differ from Plan<N>'s host tables).
-template <int N_> struct WarpPlan {
-    using B = Plan<N_>;
-    static constexpr int N = N_, T = 32, E = N_ / 32, NSTAGE = B::NSTAGE;
-    static constexpr int row_swz = B::row_swz, row_sh = B::row_sh, col_c = B::col_c, col_ps = B::col_ps;
-    static constexpr bool PK = true, PKMUL = false, OWN_TW = false;
-    static constexpr int radix(int s) { return B::radix(s); }
+// Two-stage lines of the mixed sides, N = 24 RB (384: RB = 16, 768: RB = 32).  No
+// thread count divides the work of both stages, so the stages own different elements:
+// the radix-RB stage is 24 butterflies on elements j + 24 r (j < 24, some threads
+// idle), the radix-24 stage RB butterflies on j + RB r (every thread one).  A transform
+// goes from the first ownership to the second (to24: radix RB, then 24) or back
+// (from24: radix 24, then RB), so a pass transforms, works pointwise on 24 elements a
+// thread and transforms back in the ownership it started with, with one exchange per
+// transform.  The exchange runs in the line's own slots with padded pitches: RB + 1
+// after the radix-RB stage, 25 after the radix-24 stage, both conflict-free for 16
+// consecutive butterflies (rows) and for 4 rows x 4 columns or 2 x 8 (columns), as is
+// the natural order; the line needs SLOTS >= N slots for them.
+template <int N_> struct Mixed {
+    static constexpr int N = N_, RB = N_ / 24, T = RB, E = 24;
+    static constexpr int QV_ROW = RB == 16 ? 2 : 1;  // radix-RB butterflies a thread holds
+    static constexpr int PA = RB + 1, PB = 25, SLOTS = 24 * PA > RB * PB ? 24 * PA : RB * PB;
+    static constexpr bool PK = true;
+    static_assert(N == 384 || N == 768, "sides of the two-stage mixed plans");
 };
-// The mixed sides one warp per line with fewer stages than Plan<N>, the radix
-// 6 / 12 stage last so the spans before it are powers of two, and an exchange
-// swizzle i ^ ((i >> sh) & 15) under which every exchange is conflict-free (a
-// CPU bank model of the half-warp wavefronts checked each one): 384 = 8 x 8 x 6
-// on half-warp lines (16 threads x 24 elements, two lines per warp), 768 = 8 x 8
-// x 12 on warp lines (32 threads x 24 elements).
-template <> struct WarpPlan<384> {  // half-warp lines (two per warp)
-    static constexpr int N = 384, T = 16, E = 24, NSTAGE = 3;
-    static constexpr int row_swz = 1, row_sh = 3, col_c = 4, col_ps = 30;
-    static constexpr bool PK = true, PKMUL = false, OWN_TW = true;
-    static constexpr int radix(int s) { return s < 2 ? 8 : 6; }
-};
-template <> struct WarpPlan<768> {
-    static constexpr int N = 768, T = 32, E = 24, NSTAGE = 3;
-    static constexpr int row_swz = 1, row_sh = 3, col_c = 4, col_ps = 30;
-    static constexpr bool PK = true, PKMUL = false, OWN_TW = true;
-    static constexpr int radix(int s) { return s < 2 ? 8 : 12; }
-};
+// Slot access: `at(i)` is the shared address of slot i of the thread's line.  v: QV
+// butterflies of RB elements, vj their numbers (>= 24: none), u: 24 elements of
+// butterfly uj; t24[r][k] = w^(r k), k < RB and tb[r][k], k < 24 (w = exp(2 pi i / N)).
+template <class M, int DIR, int QV, class AtV, class AtU, class Sync>
+__device__ __forceinline__ void mixed_to24(float2 (&v)[QV * M::RB], float2 (&u)[24], const int (&vj)[QV], int uj,
+                                           const AtV &atv, const AtU &atu, const float2 *__restrict__ t24,
+                                           const Sync &sync) {
+#pragma unroll
+    for (int q = 0; q < QV; ++q)
+        if (vj[q] < 24) dft<M::RB, DIR, M::PK>(v + q * M::RB);
+    sync();  // previous readers are done
+#pragma unroll
+    for (int q = 0; q < QV; ++q)
+        if (vj[q] < 24) {
+            const uint32_t at = atv(q, vj[q] * M::PA);
+#pragma unroll
+            for (int r = 0; r < M::RB; ++r) sts_f2(at + atv.step() * r, v[q * M::RB + r]);
+        }
+    sync();
+    const uint32_t at = atu(uj);
+#pragma unroll
+    for (int r = 0; r < 24; ++r) {
+        u[r] = lds_f2(at + atu.step() * (M::PA * r));
+        if (r) {
+            float2 w = t24[r * M::RB + uj];
+            if constexpr (DIR < 0) w.y = -w.y;
+            u[r] = c_mul(u[r], w);
+        }
+    }
+    dft<24, DIR, M::PK>(u);
+}
+template <class M, int DIR, int QV, class AtV, class AtU, class Sync>
+__device__ __forceinline__ void mixed_from24(float2 (&u)[24], float2 (&v)[QV * M::RB], const int (&vj)[QV], int uj,
+                                             const AtV &atv, const AtU &atu, const float2 *__restrict__ tb,
+                                             const Sync &sync) {
+    dft<24, DIR, M::PK>(u);
+    sync();  // previous readers are done
+    const uint32_t at = atu(uj * M::PB);
+#pragma unroll
+    for (int r = 0; r < 24; ++r) sts_f2(at + atu.step() * r, u[r]);
+    sync();
+#pragma unroll
+    for (int q = 0; q < QV; ++q)
+        if (vj[q] < 24) {
+            const uint32_t at = atv(q, vj[q]);
+#pragma unroll
+            for (int r = 0; r < M::RB; ++r) {
+                float2 x = lds_f2(at + atv.step() * (M::PB * r));
+                if (r) {
+                    float2 w = tb[r * 24 + vj[q]];
+                    if constexpr (DIR < 0) w.y = -w.y;
+                    x = c_mul(x, w);
+                }
+                v[q * M::RB + r] = x;
+            }
+            dft<M::RB, DIR, M::PK>(v + q * M::RB);
+        }
+}
 
 }  // namespace msl

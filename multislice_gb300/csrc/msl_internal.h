@@ -55,7 +55,7 @@ enum RowFlags {
     ROW_INV = 4,     // exp(-i) line transform
     ROW_TRANS = 8,   // multiply by trans[ix][iy]
     ROW_FWD = 16,    // exp(+i) line transform
-    ROW_ACCUM = 32,  // accum[line][iy] += accum_w * |psi|^2 (FP64)
+    ROW_ACCUM = 32,  // add the images' |psi|^2 onto accum (FP64; RowArgs::nimg)
     ROW_NOSTORE = 64 // do not write the wave back
 };
 
@@ -71,11 +71,10 @@ struct RowArgs {
     int flags;
     float scale;           // multiplies the output when != 1
     int *err;              // set to 1 when a bounded wait gives up (may be null)
-    double *accum;         // [nlines][ny] (ROW_ACCUM)
-    double accum_w;
-    // many images onto one accumulator (ROW_LOAD [| ROW_INV] | ROW_ACCUM | ROW_NOSTORE):
-    // image i of nimg adds accum_wt[(img0 + i) % nw] * |psi|^2 to accum[nx][ny], in order
-    int nimg, img0, nw;        // nimg = 0: one image per accumulator, accum_w
+    // images onto one accumulator (ROW_LOAD [| ROW_INV] | ROW_ACCUM | ROW_NOSTORE): image i
+    // of nimg adds accum_wt[(img0 + i) % nw] * |psi|^2 to accum[nx][ny], in order
+    double *accum;
+    int nimg, img0, nw;
     const double *accum_wt;
     const float2 *const *trans_b;  // per-image transmission rows (replaces trans when set)
     bool shared;           // other streams' kernels run beside this one

@@ -167,11 +167,6 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) row_pass_kernel(RowArgs a)
             }
             if constexpr (IMG) {
                 add_image<T>(sum, v, a, img, a.accum + (size_t)(line % a.nx) * N + t);
-            } else if (a.flags & ROW_ACCUM) {
-#pragma unroll
-                for (int e = 0; e < E; ++e)
-                    a.accum[base + t + T * e] +=
-                        a.accum_w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
             }
             if (!(a.flags & ROW_NOSTORE)) {
 #pragma unroll
@@ -671,6 +666,146 @@ __global__ void __launch_bounds__(ColHalfCfg<L>::THREADS, 1)
     }
 }
 
+// exp(2 pi i r k / N) at [r][k], r < 24, k < RB, then r < RB, k < 24
+template <int N> __device__ __forceinline__ void mixed_tables(float2 *t) {
+    constexpr int RB = Mixed<N>::RB;
+    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) {
+        const int j = i % N, m = i < N ? (j / RB) * (j % RB) : (j / 24) * (j % 24);
+        float sn, cn;
+        sincospif((float)(2 * m) / (float)N, &sn, &cn);
+        t[i] = make_float2(cn, sn);
+    }
+}
+
+// ---------------------------------------- two-stage column pass, 384 and 768
+// Columns on the Mixed plans: a CTA of four warps per tile of C columns x N rows (8 at
+// 384, 4 at 768: RB threads per column), fed by 2D TMA into a two-slot ring; the slots
+// have the exchange's padded rows (Mixed::SLOTS), and a half-warp covers 2 x 8 or 4 x 4
+// rows x columns, conflict-free in every access.  In the radix-RB stages the warps past
+// butterfly 24 are idle.  One exchange per transform, seven CTA barriers a tile (eleven
+// with the three-stage plans), six shared-memory accesses an element (ten).
+// 512 waves of 384^2: 0.251 ms a pass (0.275 before, 72 % of HBM); 128 of 768^2: 0.278
+// (0.314, 65 %).  Bound by latency as the rows, and by the barriers.
+template <int N> struct ColMixedCfg {
+    using M = Mixed<N>;
+    static constexpr int THREADS = 128, NWARP = 4, C = THREADS / M::RB, QV = (24 + M::RB - 1) / M::RB, MINB = 3;
+    static constexpr int BOXR = N / (N / 256 + 1), NBOX = N / BOXR;  // 192 or 256 rows per box
+    static constexpr uint32_t SLOT = sizeof(float2) * M::SLOTS * C;
+    static constexpr size_t OFF_T = 2 * SLOT, OFF_RED = OFF_T + sizeof(float2) * 2 * N;
+    static constexpr size_t OFF_BAR = OFF_RED + sizeof(double) * NWARP * kMaxDet;
+    static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * 2 + 128;
+    static_assert(BOXR <= 256 && BOXR * NBOX == N && SLOT % 128 == 0, "TMA boxes tile the column");
+};
+
+template <int N>
+__global__ void __launch_bounds__(128, ColMixedCfg<N>::MINB)
+    col_mixed_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap mapo, ColArgs a) {
+    using Cfg = ColMixedCfg<N>;
+    using M = Mixed<N>;
+    constexpr int C = Cfg::C, RB = M::RB, QV = Cfg::QV;
+    extern __shared__ unsigned char smraw[];
+    unsigned char *base = smraw + ((128u - (smem_u32(smraw) & 127u)) & 127u);
+    float2 *t24 = reinterpret_cast<float2 *>(base + Cfg::OFF_T), *tb = t24 + N;
+    double *red = reinterpret_cast<double *>(base + Cfg::OFF_RED);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR);
+    const int tid = threadIdx.x, c = tid % C, uj = tid / C;
+    int vj[QV];
+#pragma unroll
+    for (int q = 0; q < QV; ++q) vj[q] = uj + RB * q;
+    mixed_tables<N>(t24);
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    const bool store = (a.flags & COL_STORE) != 0;
+    const int tpi = a.ny / C, ntiles = a.batch * tpi;
+    const int nmine = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    auto ctasync = [&]() { __syncthreads(); };
+    pass_begin();
+    int issued = 0;
+    auto issue = [&](int k) {  // thread 0 only
+        const int tile = blockIdx.x + k * gridDim.x, b = tile / tpi, ty = tile % tpi, s = k & 1;
+        fence_proxy_async();
+        mbar_arrive_expect_tx(&bar[s], (uint32_t)(sizeof(float2) * N * C));
+#pragma unroll
+        for (int q = 0; q < Cfg::NBOX; ++q)
+            tma_load_2d(base + s * Cfg::SLOT + sizeof(float2) * q * Cfg::BOXR * C, &map, ty * C,
+                        col_source(a, b) * N + q * Cfg::BOXR, &bar[s]);
+        issued = k + 1;
+    };
+    if (tid == 0 && nmine > 0) issue(0);
+    int k = 0;
+    bool ok = true;
+    for (; k < nmine; ++k) {
+        const int tile = blockIdx.x + k * gridDim.x, b = tile / tpi, ty = tile % tpi, s = k & 1, iy = ty * C + c;
+        if (tid == 0 && k + 1 < nmine) {
+            if (store) tma_wait_read<0>();  // the store of tile k-1 has read the other slot
+            issue(k + 1);
+        }
+        const bool got = mbar_wait_bounded(&bar[s], (uint32_t)((k >> 1) & 1), kWaitLimit);
+        if (__syncthreads_or(!got)) {
+            ok = false;
+            break;
+        }
+        struct At {
+            uint32_t a;
+            __device__ uint32_t operator()(int, int i) const { return a + step() * (uint32_t)i; }
+            __device__ uint32_t operator()(int i) const { return a + step() * (uint32_t)i; }
+            __device__ static constexpr uint32_t step() { return 8u * C; }
+        } at = {smem_u32(base + s * Cfg::SLOT) + 8u * (uint32_t)c};
+        float2 v[QV * RB], u[24];
+        if (a.flags & COL_FWD) {
+#pragma unroll
+            for (int q = 0; q < QV; ++q)
+                if (vj[q] < 24) {
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) v[q * RB + r] = lds_f2(at(vj[q]) + at.step() * (24u * r));
+                }
+            mixed_to24<M, +1, QV>(v, u, vj, uj, at, at, t24, ctasync);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 24; ++r) u[r] = lds_f2(at(uj) + at.step() * (uint32_t)(RB * r));
+        }
+        if (a.flags & COL_PROP) col_propagate<M>(u, a, b, iy, uj);
+        if (a.flags & COL_CTF) col_ctf<M>(u, a, b, iy, uj);
+        if (a.flags & COL_DETECT) col_detect<M, Cfg::NWARP>(u, a, b, iy, uj, ty, tpi, red);
+        if (a.flags & COL_INV) mixed_from24<M, -1, QV>(u, v, vj, uj, at, at, tb, ctasync);
+        if (store) {
+            __syncthreads();  // every thread is done reading the slot
+            if (a.flags & COL_INV) {
+#pragma unroll
+                for (int q = 0; q < QV; ++q)
+                    if (vj[q] < 24) {
+#pragma unroll
+                        for (int r = 0; r < RB; ++r) sts_f2(at(vj[q]) + at.step() * (24u * r), v[q * RB + r]);
+                    }
+            } else {
+#pragma unroll
+                for (int r = 0; r < 24; ++r) sts_f2(at(uj) + at.step() * (uint32_t)(RB * r), u[r]);
+            }
+            fence_proxy_async();
+            __syncthreads();
+            if (tid == 0) {
+#pragma unroll
+                for (int q = 0; q < Cfg::NBOX; ++q)
+                    tma_store_2d(&mapo, ty * C, b * N + q * Cfg::BOXR, base + s * Cfg::SLOT + sizeof(float2) * q * Cfg::BOXR * C);
+                tma_commit();
+            }
+        } else {
+            __syncthreads();  // the slot is free before the load of tile k + 2 lands in it
+        }
+    }
+    if (tid == 0) {
+        if (store) tma_wait_all();
+        if (!ok) {
+            if (a.err) atomicExch(a.err, 1);
+            for (int j = k; j < issued; ++j) mbar_wait_bounded(&bar[j & 1], (uint32_t)((j >> 1) & 1), kWaitLimit);
+        }
+    }
+}
+
 // ---------------------------------------------------- TMA-fed row pass
 // Persistent kernel, MINB CTAs per SM, TH threads = L lines x T threads.  Tiles
 // of L consecutive lines (L * N * 8 bytes, contiguous) arrive by TMA into a ring
@@ -770,11 +905,6 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, IMG ? 1 : MINB)
         }
         if constexpr (IMG) {
             add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
-        } else if (a.flags & ROW_ACCUM) {
-            double *acc = a.accum + (size_t)line * N;
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                acc[t + T * e] += a.accum_w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
         }
         const bool st = !(a.flags & ROW_NOSTORE);
         __syncthreads();  // every thread is done reading bs
@@ -806,160 +936,150 @@ __global__ void __launch_bounds__(RowTmaCfg<N, TH>::THREADS, IMG ? 1 : MINB)
 }
 
 
-// ---------------------- warp-per-line row pass (half-warp lines at 384)
-// Persistent kernel in which every warp owns whole lines (one, or two
-// half-warp lines when the plan has 16 threads per line): it streams them
-// through its own two- or three-slot ring in shared memory with 1D bulk copies
-// (cp.async.bulk) and its own mbarriers, and the line transforms exchange
-// through that ring with warp-level synchronisation only.  No CTA-wide barrier
-// runs after the prologue, so a warp waiting on its exchange or its next line
-// never holds up the others.
-template <class A> __device__ __forceinline__ A make_row_addr(float2 *buf);
-template <> __device__ __forceinline__ RowXorLin<WarpPlan<256>> make_row_addr(float2 *buf) {
-    return RowXorLin<WarpPlan<256>>{smem_u32(buf)};
-}
-template <> __device__ __forceinline__ RowXorLin<WarpPlan<512>> make_row_addr(float2 *buf) {
-    return RowXorLin<WarpPlan<512>>{smem_u32(buf)};
-}
-template <> __device__ __forceinline__ RowXorAddr<WarpPlan<384>> make_row_addr(float2 *buf) {
-    return RowXorAddr<WarpPlan<384>>{buf};
-}
-template <> __device__ __forceinline__ RowXorAddr<WarpPlan<768>> make_row_addr(float2 *buf) {
-    return RowXorAddr<WarpPlan<768>>{buf};
-}
-
-template <int N> struct RowWarpCfg {
-    using P = WarpPlan<N>;
-    static constexpr int LPW = 32 / P::T;  // lines per warp: 1, or 2 for half-warp lines
-    static constexpr int W = 8, THREADS = 32 * W, NBUF = (N == 512 || N == 768 || LPW > 1) ? 2 : 3;
-    static constexpr int MINB = N == 512 ? 3 : P::E <= 8 ? 3 : 2;
-    static constexpr size_t LINE = sizeof(float2) * N, UNIT = LPW * LINE;
-    // power-of-two sides address their exchanges xor-linearly (RowXorLin), which
-    // needs every line buffer aligned to its size
-    static constexpr bool XL = (N & (N - 1)) == 0;
-    static constexpr uint32_t ALIGN = XL ? (uint32_t)LINE : 128u;
-    static constexpr size_t OFF_TW = (size_t)W * NBUF * UNIT;
-    static constexpr size_t OFF_BAR = OFF_TW + ((sizeof(float2) * plan_tw_size<P>() + 15) / 16) * 16;
-    static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * W * NBUF + ALIGN;
-    static_assert(P::T == 32 || P::T == 16, "warp- or half-warp-owned lines");
+// ------------------------------------------- two-stage row pass, 384 and 768
+// Rows on the Mixed plans: every warp owns whole lines (two at 384, one at 768), streamed
+// through its own two-slot ring by 1D bulk copies; one exchange per transform in the
+// line's slot, warp synchronisation only.  The three-stage plans these sides had before
+// (8 x 8 x 6 and 8 x 8 x 12) moved each element through shared memory ten times a pass,
+// which took all of its bandwidth; now six times.
+// 512 waves of 384^2: 0.233 ms a pass (0.273 before, 78 % of HBM); 128 of 768^2: 0.256
+// (0.281, 71 %).  Bound by latency at 12 warps an SM (160-168 registers): issue 48 %.
+template <int N> struct RowMixedCfg {
+    using M = Mixed<N>;
+    static constexpr int W = 4, THREADS = 32 * W, LPW = 32 / M::RB, MINB = 3;
+    static constexpr size_t SLOT = sizeof(float2) * LPW * M::SLOTS;  // a unit of LPW lines
+    static constexpr size_t OFF_T = W * 2 * SLOT, OFF_BAR = OFF_T + sizeof(float2) * 2 * N;
+    static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * W * 2 + 128;  // + base alignment
+    static_assert(sizeof(float2) * M::SLOTS % 16 == 0 && (LPW == 1 || M::SLOTS % 16 == 8),
+                  "bulk copies land on 16 bytes; a second line shifts by half the banks");
 };
-
 template <int N, bool IMG>
-__global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, IMG ? 1 : RowWarpCfg<N>::MINB) row_warp_kernel(RowArgs a) {
-    using Cfg = RowWarpCfg<N>;
-    using P = WarpPlan<N>;
-    constexpr int E = P::E, T = P::T, LPW = Cfg::LPW, NBUF = Cfg::NBUF, W = Cfg::W, TW = plan_tw_size<P>();
-    constexpr uint32_t AL = Cfg::ALIGN;
+__global__ void __launch_bounds__(RowMixedCfg<N>::THREADS, IMG ? 1 : RowMixedCfg<N>::MINB) row_mixed_kernel(RowArgs a) {
+    using Cfg = RowMixedCfg<N>;
+    using M = Mixed<N>;
+    constexpr int RB = M::RB, QV = M::QV_ROW, LPW = Cfg::LPW, W = Cfg::W, S = M::SLOTS;
     extern __shared__ unsigned char smraw[];
-    unsigned char *base = smraw + ((AL - (smem_u32(smraw) & (AL - 1u))) & (AL - 1u));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane / T, t = lane % T;
-    float2 *ring = reinterpret_cast<float2 *>(base) + (size_t)warp * NBUF * LPW * N;
-    float2 *tw = reinterpret_cast<float2 *>(base + Cfg::OFF_TW);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR) + warp * NBUF;
-    if constexpr (P::OWN_TW) {  // stage s >= 1: [r][k] = exp(2 pi i r k / (NS R)), NS = span before s
-#pragma unroll
-        for (int st = 1; st < P::NSTAGE; ++st) {
-            const int R = P::radix(st), NS = plan_span<P>(st), off = plan_tw_offset<P>(st);
-            for (int i = threadIdx.x; i < R * NS; i += Cfg::THREADS) {
-                float sn, cn;
-                sincospif((float)(2 * (i / NS) * (i % NS)) / (float)(NS * R), &sn, &cn);
-                tw[off + i] = make_float2(cn, sn);
-            }
-        }
-    } else {
-        for (int i = threadIdx.x; i < TW; i += Cfg::THREADS) tw[i] = a.tw[i];
-    }
+    unsigned char *base = smraw + ((128u - (smem_u32(smraw) & 127u)) & 127u);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *ring = base + warp * 2 * Cfg::SLOT;
+    float2 *t24 = reinterpret_cast<float2 *>(base + Cfg::OFF_T), *tb = t24 + N;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR) + warp * 2;
+    mixed_tables<N>(t24);
     if (lane == 0) {
-        for (int s = 0; s < NBUF; ++s) mbar_init(&bar[s], 1);
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
         mbar_fence_init();
     }
     __syncthreads();  // the only CTA barrier: tables and barriers are ready
     const bool load = (a.flags & ROW_LOAD) != 0, store = !(a.flags & ROW_NOSTORE);
-    const int nunits = (IMG ? a.nx : a.nlines) / LPW;  // units of LPW consecutive lines, one per warp at a time
+    const int nunits = (IMG ? a.nx : a.nlines) / LPW;
     const int G = gridDim.x * W, gw = spread_id(warp, W, a.shared);
     const int nmine = (gw < nunits ? (nunits - gw + G - 1) / G : 0) * (IMG ? a.nimg : 1);
     auto unit_of = [&](int k) {
         if constexpr (IMG) return gw + k / a.nimg * G + k % a.nimg * nunits;
         else return gw + k * G;
     };
-    [[maybe_unused]] double sum[IMG ? E : 1];
+    [[maybe_unused]] double sum[IMG ? 24 : 1];
+    // this lane's radix-24 butterfly and its radix-RB butterflies, and their lines
+    const int lu = lane / RB, uj = lane % RB;
+    int vj[QV], lv[QV];
+#pragma unroll
+    for (int q = 0; q < QV; ++q) {
+        const int b = lane + 32 * q;
+        lv[q] = b / 24 < LPW ? b / 24 : 0;
+        vj[q] = b / 24 < LPW ? b % 24 : 24;
+    }
     pass_begin();
     int issued = 0;
     auto issue = [&](int k) {  // lane 0 only
-        const int unit = unit_of(k), s = k % NBUF;
+        const int s = k & 1;
+        const float2 *src = a.in + (size_t)unit_of(k) * LPW * N;
         fence_proxy_async();
-        mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::UNIT);
-        bulk_load(ring + (size_t)s * LPW * N, a.in + (size_t)unit * LPW * N, (uint32_t)Cfg::UNIT, &bar[s]);
+        mbar_arrive_expect_tx(&bar[s], (uint32_t)(LPW * N * sizeof(float2)));
+#pragma unroll
+        for (int l = 0; l < LPW; ++l)
+            bulk_load(ring + s * Cfg::SLOT + l * S * sizeof(float2), src + l * N, (uint32_t)(N * sizeof(float2)), &bar[s]);
         issued = k + 1;
     };
-    if (load && lane == 0)
-        for (int k = 0; k < NBUF - 1 && k < nmine; ++k) issue(k);
+    if (load && lane == 0 && nmine > 0) issue(0);
     int k = 0;
     bool ok = true;
     for (; k < nmine; ++k) {
-        const int unit = unit_of(k), s = k % NBUF, line = LPW * unit + h;
-        float2 *slot = ring + (size_t)s * LPW * N;
-        float2 *buf = slot + (size_t)h * N;
-        using Addr = typename std::conditional<Cfg::XL, RowXorLin<P>, RowXorAddr<P>>::type;
-        Addr ad = make_row_addr<Addr>(buf);
-        const float2 *trow = (a.flags & ROW_TRANS)
-                                 ? (a.trans_b ? a.trans_b[line / a.nx] : a.trans) + (size_t)(line % a.nx) * N
-                                 : nullptr;
-        if (!load && store && lane == 0) tma_wait_read<NBUF - 1>();  // the store of line k-NBUF left buf
-        if constexpr (NBUF == 2) {
-            // two buffers: the next line goes into the buffer of line k-1 as soon as
-            // that line's store has read it, so it loads while line k is transformed
-            if (load && lane == 0 && k + 1 < nmine) {
-                if (store) tma_wait_read<0>();
-                issue(k + 1);
-            }
+        const int s = k & 1, unit = unit_of(k), line = LPW * unit + lu;
+        const uint32_t slot = smem_u32(ring + s * Cfg::SLOT);
+        struct At {
+            uint32_t a[QV];
+            __device__ uint32_t operator()(int q, int i) const { return a[q] + 8u * (uint32_t)i; }
+            __device__ static constexpr uint32_t step() { return 8u; }
+        } atv;
+#pragma unroll
+        for (int q = 0; q < QV; ++q) atv.a[q] = slot + 8u * (uint32_t)(lv[q] * S);
+        struct AtU {
+            uint32_t a;
+            __device__ uint32_t operator()(int i) const { return a + 8u * (uint32_t)i; }
+            __device__ static constexpr uint32_t step() { return 8u; }
+        } atu = {slot + 8u * (uint32_t)(lu * S)};
+        if (!load && store && lane == 0) tma_wait_read<1>();  // the store of unit k-2 left the slot
+        if (load && lane == 0 && k + 1 < nmine) {
+            if (store) tma_wait_read<0>();  // the store of unit k-1 has read the other slot
+            issue(k + 1);
         }
-        float2 v[E];
         if (load) {
-            const bool got = mbar_wait_bounded(&bar[s], (uint32_t)((k / NBUF) & 1), kWaitLimit);
+            const bool got = mbar_wait_bounded(&bar[s], (uint32_t)((k >> 1) & 1), kWaitLimit);
             if (__any_sync(0xffffffffu, !got)) {
                 ok = false;
                 break;
             }
+        }
+        float2 v[QV * RB], u[24];
+        if (load && (a.flags & ROW_INV)) {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = buf[t + T * e];
+            for (int q = 0; q < QV; ++q)
+                if (vj[q] < 24) {
+                    const uint32_t at = atv(q, vj[q]);
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) v[q * RB + r] = lds_f2(at + 8u * 24u * r);
+                }
+            mixed_to24<M, -1, QV>(v, u, vj, uj, atv, atu, t24, WarpSync());
+        } else if (load) {
+#pragma unroll
+            for (int r = 0; r < 24; ++r) u[r] = lds_f2(atu(uj) + 8u * (uint32_t)RB * r);
         } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = make_float2(1.f, 0.f);
+            for (int r = 0; r < 24; ++r) u[r] = make_float2(1.f, 0.f);
         }
-        if (a.flags & ROW_INV) fft_line<P, -1, 0, true>(v, t, ad, tw);
         if (a.flags & ROW_TRANS) {
+            const float2 *trow = (a.trans_b ? a.trans_b[line / a.nx] : a.trans) + (size_t)(line % a.nx) * N + uj;
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = c_mul(v[e], __ldg(trow + t + T * e));
+            for (int r = 0; r < 24; ++r) u[r] = c_mul(u[r], __ldg(trow + RB * r));
         }
-        if (a.flags & ROW_FWD) fft_line<P, +1, 0, true>(v, t, ad, tw);
-        if (a.scale != 1.0f) {
-#pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
-        }
-        if constexpr (IMG) {
-            add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
-        } else if (a.flags & ROW_ACCUM) {
-            double *acc = a.accum + (size_t)line * N;
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                acc[t + T * e] += a.accum_w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
-        }
-        if (store) {
+        if constexpr (IMG) add_image<RB>(sum, u, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + uj);
+        if (a.flags & ROW_FWD) {
+            mixed_from24<M, +1, QV>(u, v, vj, uj, atv, atu, tb, WarpSync());
             __syncwarp();  // every lane is done reading the slot
 #pragma unroll
-            for (int e = 0; e < E; ++e) buf[t + T * e] = v[e];
+            for (int q = 0; q < QV; ++q)
+                if (vj[q] < 24) {
+                    const uint32_t at = atv(q, vj[q]);
+#pragma unroll
+                    for (int r = 0; r < RB; ++r)
+                        sts_f2(at + 8u * 24u * r, a.scale != 1.0f ? c_scale(v[q * RB + r], a.scale) : v[q * RB + r]);
+                }
+        } else if (store) {
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 24; ++r)
+                sts_f2(atu(uj) + 8u * (uint32_t)RB * r, a.scale != 1.0f ? c_scale(u[r], a.scale) : u[r]);
+        }
+        if (store) {
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
-                bulk_store(a.out + (size_t)unit * LPW * N, slot, (uint32_t)Cfg::UNIT);
+#pragma unroll
+                for (int l = 0; l < LPW; ++l)
+                    bulk_store(a.out + ((size_t)unit * LPW + l) * N, ring + s * Cfg::SLOT + l * S * sizeof(float2),
+                               (uint32_t)(N * sizeof(float2)));
                 tma_commit();
-            }
-        }
-        if constexpr (NBUF == 3) {
-            if (load && lane == 0 && k + NBUF - 1 < nmine) {
-                if (store) tma_wait_read<1>();  // the store of line k-1 has left its buffer
-                issue(k + NBUF - 1);            // into buffer (k + 2) % 3
             }
         }
         __syncwarp();
@@ -968,10 +1088,24 @@ __global__ void __launch_bounds__(RowWarpCfg<N>::THREADS, IMG ? 1 : RowWarpCfg<N
         if (store) tma_wait_all();
         if (!ok) {
             if (a.err) atomicExch(a.err, 1);
-            for (int j = k; j < issued; ++j)
-                mbar_wait_bounded(&bar[j % NBUF], (uint32_t)((j / NBUF) & 1), kWaitLimit);
+            for (int j = k; j < issued; ++j) mbar_wait_bounded(&bar[j & 1], (uint32_t)((j >> 1) & 1), kWaitLimit);
         }
     }
+}
+
+template <int N, bool IMG> static cudaError_t row_mixed_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
+    using Cfg = RowMixedCfg<N>;
+    static KernelSetup ks;
+    int per_sm = 0;
+    cudaError_t e = ks.get(row_mixed_kernel<N, IMG>, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
+    if (e != cudaSuccess) return e;
+    const int units = spread_units((IMG ? a.nx : a.nlines) / Cfg::LPW, Cfg::W, a.shared);
+    int grid = nsm * per_sm < units ? nsm * per_sm : units;
+    if (grid < 1) grid = 1;
+    return launch_pass(row_mixed_kernel<N, IMG>, grid, Cfg::THREADS, Cfg::SMEM, s, !IMG && !a.shared, a);
+}
+template <int N> static cudaError_t row_mixed_launch(const RowArgs &a, cudaStream_t s, int nsm) {
+    return a.nimg ? row_mixed_launch_v<N, true>(a, s, nsm) : row_mixed_launch_v<N, false>(a, s, nsm);
 }
 
 // ------------------------------------- two-stage row pass, 256 / 512 / 1024
@@ -1073,12 +1207,6 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
         if (a.scale != 1.0f) {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = c_scale(v[e], a.scale);
-        }
-        if (a.flags & ROW_ACCUM) {
-            double *acc = a.accum + (size_t)line * N;
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                acc[t + T * e] += a.accum_w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
         }
         if (store) {
             __syncwarp();  // every lane is done reading the slot
@@ -1343,11 +1471,6 @@ __global__ void __launch_bounds__(RowPairCfg::THREADS, IMG ? 1 : RowPairCfg::MIN
         }
         if constexpr (IMG) {
             add_image<T>(sum, v, a, k % a.nimg, a.accum + (size_t)(line % a.nx) * N + t);
-        } else if (a.flags & ROW_ACCUM) {
-            double *acc = a.accum + (size_t)line * N;
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                acc[t + T * e] += a.accum_w * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
         }
         pairsync();  // both warps are done reading the slot (and, without a load, the old store left it)
         if (store) {
@@ -1627,6 +1750,34 @@ static bool tma_eligible(const ColArgs &a) {
     return encode_fn() != nullptr;
 }
 
+// Tensor maps of a column pass, boxes of C columns x boxr rows; loads and stores use one
+// map unless results fan out.
+static bool col_maps(const ColArgs &a, int n, int c, int boxr, CUtensorMap *load, CUtensorMap *store) {
+    auto encode = [&](CUtensorMap *m, const void *p, int images) {
+        const uint64_t dims[2] = {(uint64_t)a.ny, (uint64_t)images * n};
+        const uint64_t strides[1] = {(uint64_t)a.ny * sizeof(float2)};
+        const uint32_t box[2] = {(uint32_t)c, (uint32_t)boxr};
+        return encode_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p, dims, strides, box,
+                                 CU_TENSOR_MAP_SWIZZLE_NONE);
+    };
+    if (!encode(store, a.out, a.batch)) return false;
+    *load = *store;
+    return !a.fan || encode(load, a.in, (a.img0 + a.batch - 1) / a.fan + 1);
+}
+
+template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStream_t s, int nsm) {
+    using Cfg = ColMixedCfg<N>;
+    static KernelSetup ks;
+    int per_sm = 0;
+    cudaError_t e = ks.get(col_mixed_kernel<N>, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
+    if (e != cudaSuccess) return e;
+    CUtensorMap map, mapo;
+    if (!col_maps(a, N, Cfg::C, Cfg::BOXR, &map, &mapo)) return cudaErrorInvalidValue;
+    const int ntiles = a.batch * (a.ny / Cfg::C);
+    const int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
+    return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, mapo, a);
+}
+
 template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs &a, cudaStream_t s, int nsm) {
     using Cfg = ColTmaCfg<PL>;
     constexpr int N = PL::N;
@@ -1636,18 +1787,8 @@ template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs 
         cudaError_t e = ks.get(col_tma_kernel<PL, MINB>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
         if (e != cudaSuccess) return e;
     }
-    // waves as rows of columns; loads and stores use one map unless results fan out
-    auto encode = [&](CUtensorMap *m, const void *p, int images) {
-        const uint64_t dims[2] = {(uint64_t)a.ny, (uint64_t)images * N};
-        const uint64_t strides[1] = {(uint64_t)a.ny * sizeof(float2)};
-        const uint32_t box[2] = {(uint32_t)Cfg::C, (uint32_t)Cfg::BOXR};
-        return encode_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p, dims, strides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_NONE);
-    };
-    CUtensorMap mapo, map;
-    if (!encode(&mapo, a.out, a.batch)) return cudaErrorInvalidValue;
-    map = mapo;
-    if (a.fan && !encode(&map, a.in, (a.img0 + a.batch - 1) / a.fan + 1)) return cudaErrorInvalidValue;
+    CUtensorMap map, mapo;
+    if (!col_maps(a, N, Cfg::C, Cfg::BOXR, &map, &mapo)) return cudaErrorInvalidValue;
     const int ntiles = a.batch * (a.ny / Cfg::C);
     int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
     if (grid < 1) grid = 1;
@@ -1733,22 +1874,8 @@ template <int N> static cudaError_t row_tma_launch(const RowArgs &a, cudaStream_
 }
 
 
-template <int N, bool IMG> static cudaError_t row_warp_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
-    using Cfg = RowWarpCfg<N>;
-    static KernelSetup ks;
-    int per_sm = 0;
-    {
-        cudaError_t e = ks.get(row_warp_kernel<N, IMG>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
-        if (e != cudaSuccess) return e;
-    }
-    const int units = spread_units((IMG ? a.nx : a.nlines) / Cfg::LPW, Cfg::W, a.shared);
-    int grid = nsm * per_sm < units ? nsm * per_sm : units;
-    if (grid < 1) grid = 1;
-    return launch_pass(row_warp_kernel<N, IMG>, grid, Cfg::THREADS, Cfg::SMEM, s, !IMG && !a.shared, a);
-}
-
-// Warp-owned lines for the sides whose plan fits 32 threads per line.
-static bool row_warp_eligible(int ny, const RowArgs &a) {
+// Sides whose rows the fast family streams line by line (bulk copies want 16 bytes).
+static bool row_fast_eligible(int ny, const RowArgs &a) {
     if (ny != 256 && ny != 384 && ny != 512 && ny != 768 && ny != 1024 && ny != 2048) return false;
     if (a.flags & ROW_GENT) return false;
     if (((uintptr_t)a.out & 15u) || ((a.flags & ROW_LOAD) && ((uintptr_t)a.in & 15u))) return false;
@@ -1852,6 +1979,8 @@ int plan_col_c_launch(int n, const ColArgs &a) {
         ColArgs f = a;
         f.flags = (f.flags | COL_LOAD | COL_FWD) & ~COL_PROBE;
         if (fam == FAM_FAST && col_half_side(n, f)) return 4;
+        if (fam == FAM_FAST && n == 384) return ColMixedCfg<384>::C;
+        if (fam == FAM_FAST && n == 768) return ColMixedCfg<768>::C;
         switch (n) {
 #define X(N) case N: return ColPlan<N>::col_c;
             MSL_FOR_EACH_SIDE(X)
@@ -1990,9 +2119,6 @@ static TcPassArgs tc_col_args(int nx, const ColArgs &a) {
 template <class P> static cudaError_t row_two_launch(const RowArgs &a, cudaStream_t s, int nsm) {
     return a.nimg ? row_images_launch<P>(a, s, nsm) : row_two_launch_v<P>(a, s, nsm);
 }
-template <int N> static cudaError_t row_warp_launch(const RowArgs &a, cudaStream_t s, int nsm) {
-    return a.nimg ? row_warp_launch_v<N, true>(a, s, nsm) : row_warp_launch_v<N, false>(a, s, nsm);
-}
 static cudaError_t row_pair_launch(const RowArgs &a, cudaStream_t s, int nsm) {
     return a.nimg ? row_pair_launch_v<true>(a, s, nsm) : row_pair_launch_v<false>(a, s, nsm);
 }
@@ -2005,20 +2131,13 @@ cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, i
     if (fam0 == FAM_TC && row_tc_eligible(ny, a)) return launch_tc_pass(tc_row_args(ny, a), s, nsm, launches);
     ++*launches;
     const int fam = fam0 == FAM_TC ? FAM_FAST : fam0;
-    if (fam == FAM_FAST && row_warp_eligible(ny, a)) {
+    if (fam == FAM_FAST && row_fast_eligible(ny, a)) {
         switch (ny) {
-            case 256:
-                if (a.nlines % 2 == 0 && !(((uintptr_t)a.out | (uintptr_t)a.in) & 15u))
-                    return row_two_launch<HalfWarpPlan256>(a, s, nsm);
-                return row_warp_launch<256>(a, s, nsm);
-            case 384:  // half-warp lines: in pairs
-                if (a.nlines % 2 == 0) return row_warp_launch<384>(a, s, nsm);
-                break;
-            case 768: return row_warp_launch<768>(a, s, nsm);
-            case 512:
-                if (a.nlines % 2 == 0 && !(((uintptr_t)a.out | (uintptr_t)a.in) & 15u))
-                    return row_two_launch<HalfWarpPlan512>(a, s, nsm);
-                return row_warp_launch<512>(a, s, nsm);
+            // an image has an even number of rows, so lines always pair up
+            case 256: return row_two_launch<HalfWarpPlan256>(a, s, nsm);
+            case 384: return row_mixed_launch<384>(a, s, nsm);
+            case 512: return row_two_launch<HalfWarpPlan512>(a, s, nsm);
+            case 768: return row_mixed_launch<768>(a, s, nsm);
             case 1024: return row_two_launch<WarpPlan1024x2>(a, s, nsm);
             case 2048: return row_pair_launch(a, s, nsm);
             default: break;
@@ -2052,6 +2171,10 @@ cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, i
             case 512: return col_half_launch<ColHalfL512>(a, s, nsm);
             case 1024: return col_half_launch<ColPairL1024>(a, s, nsm);
             default: break;
+        }
+        if (fam == FAM_FAST && (a.flags & COL_LOAD)) {  // 384 and 768: two-stage columns for every loaded pass
+            if (nx == 384) return col_mixed_launch<384>(a, s, nsm);
+            if (nx == 768) return col_mixed_launch<768>(a, s, nsm);
         }
         switch (nx) {
 #define X(N) case N: return col_tma_launch<N>(a, s, nsm);
