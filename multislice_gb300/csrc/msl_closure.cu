@@ -20,8 +20,8 @@
 //     backward pass's ReLU mask) in the epilogue, bf16 activations out.  The same
 //     kernel computes the input gradient of these layers with the flipped,
 //     transposed weights.
-//   * conv_small_kernel: the 1 -> C and C -> 1 layers and the input gradient
-//     of the last layer on the CUDA cores (FP32).
+//   * first_layer_kernel, last_layer_kernel, last_layer_dx_kernel: the 1 -> C and
+//     C -> 1 layers and the latter's input gradient on the CUDA cores (FP32).
 //   * dw_tc_kernel, dw_edge_kernel: weight gradients of the C -> C layers on the
 //     tensor cores and of the edge layers on the CUDA cores, FP32 partial sums per
 //     CTA reduced in a fixed order (deterministic).
@@ -62,6 +62,22 @@ inline int param_offset(int l) {
 inline int param_count() { return param_offset(kLayers); }
 
 // ------------------------------------------------------------------ helpers
+// A running sum as an unevaluated pair hi + lo (Knuth's two-sum, 48 bits): FP64 adds
+// and conversions run at a few per clock and SM here and bounded the reductions.
+struct PairSum {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float x, float tail = 0.f) {
+        const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)), tail));
+        hi = s;
+    }
+    __device__ __forceinline__ void add_square(float x) {
+        const float p = __fmul_rn(x, x);
+        add(p, fmaf(x, x, -p));
+    }
+    // (an infinite or overflowed sum has a NaN tail)
+    __device__ __forceinline__ double value() const { return isfinite(lo) ? (double)hi + (double)lo : (double)hi; }
+};
 __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
 
 // Real weight of the expanded layer: output real channel n, input real channel k.
@@ -125,12 +141,14 @@ struct Pad {
 // backward pass's ReLU mask) to bf16 through swizzled staging tiles and TMA stores.  Output row y keeps
 // its accumulator while input rows y - 1, y, y + 1 pass, in tap order, so its FP32
 // sum order is tap 0..8, channels ascending.  Eight accumulators rotate, so the
-// epilogue may lag five rows.
+// epilogue may lag five rows; it leaves them zeroed, so that no row's first product
+// needs an MMA of its own (an MMA costs some 90 cycles before its columns count: 64
+// columns 100, 192 columns 122).
 // An input tile is read from L2 three times (the shifts), not nine, and nothing but
 // TMA moves operands: what bounds it is the activations' traffic (2 x 128 bytes a
-// pixel) beside the MMA issue (12 x 96 cycles per 128 pixels).
+// pixel) beside the MMAs (12 x 122 cycles per 128 pixels, measured).
 // 16 waves of 512^2 (537 MB in, 537 MB out): 1.33 ms a layer with each tap tile copied by the threads
-// that issued its MMAs, now 0.29 ms.
+// that issued its MMAs, now 0.24 ms.
 enum Epi { EPI_BIAS_RELU = 0, EPI_MASK = 1 };
 
 constexpr size_t kWTile = 64 * 128;          // one tap's B tile: 64 rows x 128 bytes
@@ -184,6 +202,27 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// An output tile's 128 pixels of row y leave a swizzled staging tile by TMA, the first
+// and last row also to their halo rows (one thread) ...
+__device__ __forceinline__ void store_tile(const CUtensorMap *map, const void *st, int b, int y, int x0, int H) {
+    const int row = b * (H + 2) + y + 1;
+    tma_store_3d(map, 0, x0 + 1, row, st);
+    if (y == 0) tma_store_3d(map, 0, x0 + 1, row + H, st);           // halo row H
+    else if (y == H - 1) tma_store_3d(map, 0, x0 + 1, row - H, st);  // halo row -1
+    tma_commit();
+}
+// ... and an edge pixel's 64 channels to the halo columns, from the thread that holds them.
+__device__ __forceinline__ void store_halo_column(const Pad &pd, __nv_bfloat16 *out, int b, int y, int x,
+                                                  const __nv_bfloat16 *px) {
+    if (x != 0 && x != pd.W - 1) return;
+    const int xa = x == 0 ? pd.W : -1;
+    pd.each_copy(y, 1, [&](int yy, int) {
+        uint4 *h = (uint4 *)(out + pd.at(b, yy, xa) * 64);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) h[c] = *(const uint4 *)(px + c * 8);
+    });
+}
+
 __global__ void __launch_bounds__(kConvThreads, 1)
     conv_tc_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout,
                    const __nv_bfloat16 *__restrict__ wt, const float *__restrict__ bias,
@@ -226,6 +265,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
+    if (warp >= 2 && warp < 6) {  // four warps, one per lane quarter
+#pragma unroll
+        for (int i = 0; i < kAcc; ++i) tc::tmem_zero64(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64u * i);
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
     const int H = units.H, W = units.W, nunits = units.count();
     const Pad pd = {H, W};
     if (warp == 0) {
@@ -268,8 +314,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 // ascend with the tap, up to the wrap, so taps klo..khi are one or two runs
                 const uint32_t slot = 7u - ((ob + (uint32_t)(i - klo)) & 7u);
                 const int taps = khi - klo + 1, n0 = taps < 8 - (int)slot ? taps : 8 - (int)slot;
-                const uint32_t col0 = tmem + 64u * slot, id0 = tc::idesc_bf16(kTile, 64 * n0),
-                               id1 = tc::idesc_bf16(kTile, 64 * (taps - n0));
+                const uint32_t col0 = tmem + 64u * slot;
                 for (int kx = 0; kx < 3; ++kx, ++n) {
                     const uint32_t s = n % kRing;
                     if (!(ok = wait_or_quit(&full[s], (n / kRing) & 1, &failed))) break;
@@ -277,18 +322,18 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     if (tc::elect_one()) {
                         const uint64_t ad = tc::desc_sw128(saa + s * (uint32_t)kATile);
                         const uint64_t bd = tc::desc_sw128(swa + (kx * 3 + klo) * (uint32_t)kWTile);
-                        const uint64_t wrap = bd + n0 * (kWTile >> 4);  // the weights past the wrap
+                        if (n0 == 3) {  // by far the most: straight, every operand a constant step on
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {  // 16 channels: 32 bytes
-                            if (kk == 0 && kx == 0 && i < rows) {
-                                // output row i's first product overwrites its accumulator (tap 0: klo = 0)
-                                tc::mma_bf16(col0, ad, bd, tc::idesc_bf16(kTile, 64), 0u);
-                                if (n0 > 1)
-                                    tc::mma_bf16(col0 + 64u, ad, bd + (kWTile >> 4), id0 - tc::idesc_n(64), 1u);
-                            } else {
+                            for (int kk = 0; kk < 4; ++kk)  // 16 channels: 32 bytes
+                                tc::mma_bf16(col0, ad + 2 * kk, bd + 2 * kk, tc::idesc_bf16(kTile, 192), 1u);
+                        } else {
+                            const uint64_t wrap = bd + n0 * (kWTile >> 4);  // the weights past the wrap
+                            const uint32_t id0 = tc::idesc_bf16(kTile, 64 * n0), id1 = tc::idesc_bf16(kTile, 64 * (taps - n0));
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk) {
                                 tc::mma_bf16(col0, ad + 2 * kk, bd + 2 * kk, id0, 1u);
+                                if (n0 < taps) tc::mma_bf16(tmem, ad + 2 * kk, wrap + 2 * kk, id1, 1u);
                             }
-                            if (n0 < taps) tc::mma_bf16(tmem, ad + 2 * kk, wrap + 2 * kk, id1, 1u);
                         }
                         tc::mma_commit(&empty[s]);
                         if (kx == 2 && i >= 2) tc::mma_commit(&acc_full[(ob + i - 2) % kAcc]);
@@ -332,6 +377,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 tc::fence_after_sync();
                 float v[64];
                 tc::tmem_ld64(tmem + lane_base + 64u * (7u - a), v);
+                tc::tmem_zero64(tmem + lane_base + 64u * (7u - a));  // its next row adds from the first product on
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[a]);
@@ -344,23 +390,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 }
 #pragma unroll
                 for (int c = 0; c < 8; ++c) *(uint4 *)(st + tc::sw128_offset(r, c * 8)) = *(const uint4 *)(ob16 + c * 8);
-                if (x == 0 || x == W - 1) {  // the halo columns, beside the tile
-                    const int xa = x == 0 ? W : -1;
-                    pd.each_copy(y, 1, [&](int yy, int) {
-                        uint4 *h = (uint4 *)(out + pd.at(b, yy, xa) * 64);
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) h[c] = *(const uint4 *)(ob16 + c * 8);
-                    });
-                }
+                store_halo_column(pd, out, b, y, x, ob16);
                 fence_proxy_async();
                 bar_group(bar, 128);
-                if (et == 0) {
-                    const int row = b * (H + 2) + y + 1;
-                    tma_store_3d(&mout, 0, x0 + 1, row, st);
-                    if (y == 0) tma_store_3d(&mout, 0, x0 + 1, row + H, st);           // halo row H
-                    else if (y == H - 1) tma_store_3d(&mout, 0, x0 + 1, row - H, st);  // halo row -1
-                    tma_commit();
-                }
+                if (et == 0) store_tile(&mout, st, b, y, x0, H);
             }
             ob += (uint32_t)(y1 - y0);
         }
@@ -379,53 +412,58 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // or positive.
 constexpr int kEdgeWarps = 8;
 
-// (a.x, a.y) + (wr, wi) x, x given as the pairs (xr, xr), (xi, xi), m = (-wi, wr)
-__device__ __forceinline__ float2 c_mac(float2 a, float2 w, float2 m, float2 xr, float2 xi) {
-    return __fadd2_rn(a, __ffma2_rn(xr, w, __fmul2_rn(xi, m)));
+// Periodic index one step outside [0, n) at most.
+__device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : i >= n ? i - n : i; }
+
+// a + w x, scalar operations: the packed FP32 pairs run on one of the SM's two FMA pipes
+// only, at half the rate of scalar ones on both.
+__device__ __forceinline__ float2 c_mac(float2 a, float2 w, float2 x) {
+    return make_float2(__fadd_rn(a.x, fmaf(w.x, x.x, -__fmul_rn(w.y, x.y))),
+                       __fadd_rn(a.y, fmaf(w.y, x.x, __fmul_rn(w.x, x.y))));
 }
 
 // First layer: x (complex64 [B][H][W], scaled by 1/s[b]) -> h1 = CReLU(conv + b)
 // (padded bf16); the scaled input is also written as bf16 [B][H][W][2] for the
 // weight gradient when xin is given.  A warp takes runs of 32 pixels of a row: the
 // 3 x 34 inputs are scaled, rounded to bf16 (as the tensor-core layers see theirs)
-// and kept in shared memory as operand pairs, and each lane holds its channel's
-// weights in registers, so a pixel is 27 packed operations a lane and its stores
-// are two whole 64-byte halves.  16 waves of 512^2: 0.43 ms (2.2 ms with a thread
+// and kept in shared memory, and each lane holds its channel's weights in registers,
+// so a pixel is 54 operations a lane and its stores are two whole 64-byte halves.  (On the tensor cores the sums round differently, and
+// a flipped bf16 rounding here grows to 5e-4 of the output over the layers.)  16 waves of 512^2: 0.39 ms (2.2 ms with a thread
 // per pixel, whose 64 two-byte stores each touched a line of their own).
-__global__ void __launch_bounds__(32 * kEdgeWarps)
+__global__ void __launch_bounds__(32 * kEdgeWarps, 3)
     first_layer_kernel(const float2 *__restrict__ psi, const float *__restrict__ inv_s, const float *__restrict__ wl,
                        __nv_bfloat162 *__restrict__ xin, __nv_bfloat16 *__restrict__ h, int B, int H, int W) {
-    __shared__ float4 win[kEdgeWarps][3][34];  // (re, re, im, im)
+    __shared__ float2 win[kEdgeWarps][3][34];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Pad pd = {H, W};
-    float2 w[9], m[9];
+    float2 w[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
         w[t] = make_float2(bf(__float2bfloat16_rn(wl[(t * kC + lane) * 2])),
                            bf(__float2bfloat16_rn(wl[(t * kC + lane) * 2 + 1])));
-        m[t] = make_float2(-w[t].y, w[t].x);
     }
     const float2 bias = make_float2(wl[9 * kC * 2 + lane * 2], wl[9 * kC * 2 + lane * 2 + 1]);
-    const long runs = (long)B * H * (W / 32);
-    for (long u = (long)blockIdx.x * kEdgeWarps + warp; u < runs; u += (long)gridDim.x * kEdgeWarps) {
-        const int x0 = (int)(u % (W / 32)) * 32, y = (int)(u / (W / 32) % H), b = (int)(u / (W / 32) / H);
+    const unsigned rr = (unsigned)W / 32u, runs = (unsigned)B * H * rr;
+    for (unsigned u = blockIdx.x * kEdgeWarps + warp; u < runs; u += gridDim.x * kEdgeWarps) {
+        const unsigned line = u / rr;
+        const int x0 = (int)(u - line * rr) * 32, b = (int)(line / H), y = (int)line - b * H;
         const float sc = inv_s[b];
         __syncwarp();
         for (int i = lane; i < 3 * 34; i += 32) {
-            const int yy = (y + i / 34 - 1 + H) % H, xx = (x0 + i % 34 - 1 + W) % W;
+            const int yy = wrap(y + i / 34 - 1, H), xx = wrap(x0 + i % 34 - 1, W);
             const float2 v = psi[((size_t)b * H + yy) * W + xx];
-            const float xr = bf(__float2bfloat16_rn(v.x * sc)), xi = bf(__float2bfloat16_rn(v.y * sc));
-            win[warp][i / 34][i % 34] = make_float4(xr, xr, xi, xi);
+            win[warp][i / 34][i % 34] =
+                make_float2(bf(__float2bfloat16_rn(v.x * sc)), bf(__float2bfloat16_rn(v.y * sc)));
         }
         __syncwarp();
         if (xin) {
-            const float4 c = win[warp][1][1 + lane];
-            xin[((size_t)b * H + y) * W + x0 + lane] = __floats2bfloat162_rn(c.x, c.z);
+            const float2 c = win[warp][1][1 + lane];
+            xin[((size_t)b * H + y) * W + x0 + lane] = __floats2bfloat162_rn(c.x, c.y);
         }
-        const bool edge_row = y == 0 || y == H - 1;
+        const bool edge = y == 0 || y == H - 1 || x0 == 0 || x0 == W - 32;  // the run touches a halo
         __nv_bfloat16 *o = h + pd.at(b, y, x0) * 64 + lane;
         for (int x = 0; x < 32; x += 4) {
-            float4 v[3][6];
+            float2 v[3][6];
 #pragma unroll
             for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -434,21 +472,18 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
             for (int j = 0; j < 4; ++j) {
                 float2 a = bias;
 #pragma unroll
-                for (int t = 0; t < 9; ++t) {
-                    const float4 q = v[t / 3][j + t % 3];
-                    a = c_mac(a, w[t], m[t], make_float2(q.x, q.y), make_float2(q.z, q.w));
-                }
-                const __nv_bfloat16 vr = __float2bfloat16_rn(fmaxf(a.x, 0.0f)), vi = __float2bfloat16_rn(fmaxf(a.y, 0.0f));
-                const int px = x0 + x + j;
-                if (edge_row || px == 0 || px == W - 1) {
-                    pd.each_copy(y, px, [&](int yy, int xx) {
+                for (int t = 0; t < 9; ++t) a = c_mac(a, w[t], v[t / 3][j + t % 3]);
+                const __nv_bfloat162 v2 =
+                    __hmax2(__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(0.0f, 0.0f));
+                if (edge) {
+                    pd.each_copy(y, x0 + x + j, [&](int yy, int xx) {
                         __nv_bfloat16 *q = h + pd.at(b, yy, xx) * 64 + lane;
-                        q[0] = vr;
-                        q[kC] = vi;
+                        q[0] = v2.x;
+                        q[kC] = v2.y;
                     });
                 } else {
-                    o[(x + j) * 64] = vr;
-                    o[(x + j) * 64 + kC] = vi;
+                    o[(x + j) * 64] = v2.x;
+                    o[(x + j) * 64 + kC] = v2.y;
                 }
             }
         }
@@ -547,35 +582,34 @@ __global__ void __launch_bounds__(kTile)
 
 // Input gradient of the last layer, masked by h5 > 0: dh5 = mask * conv^T(g) (padded
 // bf16).  As the first layer: a lane per complex channel, runs of 32 pixels.
-__global__ void __launch_bounds__(32 * kEdgeWarps)
+__global__ void __launch_bounds__(32 * kEdgeWarps, 3)
     last_layer_dx_kernel(const float2 *__restrict__ g, const float *__restrict__ wl,
                          const __nv_bfloat16 *__restrict__ h5, __nv_bfloat16 *__restrict__ dh, int B, int H, int W) {
-    __shared__ float4 win[kEdgeWarps][3][34];
+    __shared__ float2 win[kEdgeWarps][3][34];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Pad pd = {H, W};
     // d = sum W h: dL/dhr = wr gr + wi gi, dL/dhi = -wi gr + wr gi
-    float2 w[9], m[9];
+    float2 w[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
         const float wr = bf(__float2bfloat16_rn(wl[(t * kC + lane) * 2])),
                     wi = bf(__float2bfloat16_rn(wl[(t * kC + lane) * 2 + 1]));
         w[t] = make_float2(wr, -wi);
-        m[t] = make_float2(wi, wr);
     }
-    const long runs = (long)B * H * (W / 32);
-    for (long u = (long)blockIdx.x * kEdgeWarps + warp; u < runs; u += (long)gridDim.x * kEdgeWarps) {
-        const int x0 = (int)(u % (W / 32)) * 32, y = (int)(u / (W / 32) % H), b = (int)(u / (W / 32) / H);
+    const unsigned rr = (unsigned)W / 32u, runs = (unsigned)B * H * rr;
+    for (unsigned u = blockIdx.x * kEdgeWarps + warp; u < runs; u += gridDim.x * kEdgeWarps) {
+        const unsigned line = u / rr;
+        const int x0 = (int)(u - line * rr) * 32, b = (int)(line / H), y = (int)line - b * H;
         __syncwarp();
         for (int i = lane; i < 3 * 34; i += 32) {
-            const int yy = (y + i / 34 - 1 + H) % H, xx = (x0 + i % 34 - 1 + W) % W;
-            const float2 v = g[((size_t)b * H + yy) * W + xx];
-            win[warp][i / 34][i % 34] = make_float4(v.x, v.x, v.y, v.y);
+            const int yy = wrap(y + i / 34 - 1, H), xx = wrap(x0 + i % 34 - 1, W);
+            win[warp][i / 34][i % 34] = g[((size_t)b * H + yy) * W + xx];
         }
         __syncwarp();
-        const bool edge_row = y == 0 || y == H - 1;
+        const bool edge = y == 0 || y == H - 1 || x0 == 0 || x0 == W - 32;  // the run touches a halo
         const size_t at = pd.at(b, y, x0) * 64 + lane;
         for (int x = 0; x < 32; x += 4) {
-            float4 v[3][6];
+            float2 v[3][6];
 #pragma unroll
             for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -584,16 +618,13 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
             for (int j = 0; j < 4; ++j) {
                 float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int t = 0; t < 9; ++t) {
-                    const float4 q = v[2 - t / 3][j + 2 - t % 3];  // the pixel that sees this one through tap t
-                    a = c_mac(a, w[t], m[t], make_float2(q.x, q.y), make_float2(q.z, q.w));
-                }
+                for (int t = 0; t < 9; ++t)  // the pixel that sees this one through tap t
+                    a = c_mac(a, w[t], v[2 - t / 3][j + 2 - t % 3]);
                 const size_t o = at + (size_t)(x + j) * 64;
                 const __nv_bfloat16 vr = __float2bfloat16_rn(bf(h5[o]) > 0.f ? a.x : 0.f),
                                     vi = __float2bfloat16_rn(bf(h5[o + kC]) > 0.f ? a.y : 0.f);
-                const int px = x0 + x + j;
-                if (edge_row || px == 0 || px == W - 1) {
-                    pd.each_copy(y, px, [&](int yy, int xx) {
+                if (edge) {
+                    pd.each_copy(y, x0 + x + j, [&](int yy, int xx) {
                         __nv_bfloat16 *q = dh + pd.at(b, yy, xx) * 64 + lane;
                         q[0] = vr;
                         q[kC] = vi;
@@ -744,7 +775,7 @@ __global__ void __launch_bounds__(kDwThreads, 1)
 //   first layer (wide = dy, s = x, sgn = +1):  dW[tap][n][k = c]
 //   last layer (wide = x, s = dy, sgn = -1):   dW[tap][n = c][k]
 // 36 FMAs a pixel and lane on values in registers: issue-bound, one read of the
-// wide activation.  8 waves of 256^2: 51 / 57 us (5.7 ms each on 64 x 64 tiles of zeros).
+// wide activation.  8 waves of 256^2: 48 us each (5.7 ms on 64 x 64 tiles of zeros).
 template <bool LAST>
 __global__ void __launch_bounds__(32 * kEdgeWarps)
     dw_edge_kernel(const __nv_bfloat16 *__restrict__ wide, const float2 *__restrict__ sf,
@@ -754,12 +785,13 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Pad pd = {H, W};
     float acc[9][2][2] = {}, bias[2] = {};  // [tap][narrow value][re / im half of the wide channel]
-    const long runs = (long)B * H * (W / 32);
-    for (long u = (long)blockIdx.x * kEdgeWarps + warp; u < runs; u += (long)gridDim.x * kEdgeWarps) {
-        const int x0 = (int)(u % (W / 32)) * 32, y = (int)(u / (W / 32) % H), b = (int)(u / (W / 32) / H);
+    const unsigned rr = (unsigned)W / 32u, runs = (unsigned)B * H * rr;
+    for (unsigned u = blockIdx.x * kEdgeWarps + warp; u < runs; u += gridDim.x * kEdgeWarps) {
+        const unsigned line = u / rr;
+        const int x0 = (int)(u - line * rr) * 32, b = (int)(line / H), y = (int)line - b * H;
         __syncwarp();
         for (int i = lane; i < 3 * 34; i += 32) {
-            const int yy = (y + i / 34 - 1 + H) % H, xx = (x0 + i % 34 - 1 + W) % W;
+            const int yy = wrap(y + i / 34 - 1, H), xx = wrap(x0 + i % 34 - 1, W);
             const size_t p = ((size_t)b * H + yy) * W + xx;
             win[warp][i / 34][i % 34] = LAST ? sf[p] : __bfloat1622float2(sb[p]);
         }
@@ -816,36 +848,41 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
     }
 }
 
-// The partial sums of one layer added in FP64, in a fixed order, and contracted to
+// The partial sums of one layer added in a fixed order and contracted to
 // the complex parameters: the expanded layer holds [[Wr, -Wi], [Wi, Wr]], so dWr is
 // the sum of its two Wr blocks and dWi the difference of the others; db likewise.
 // 32 parameters a block, their partials shared among kRedParts threads each (one
-// thread over all of them waited for its loads: 105 us against 29 for 152 CTAs).
+// thread over all of them waited for its loads: 105 us for 152 CTAs; FP64 sums took
+// 29, float pairs 17).
 constexpr int kRedParts = 16;
 __global__ void __launch_bounds__(32 * kRedParts)
     dw_reduce_kernel(const float *__restrict__ partial, int nblocks, int co, int ci, float *__restrict__ g) {
-    __shared__ double part[kRedParts][4][32];
+    __shared__ float2 part[kRedParts][4][32];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, nw = 9 * co * ci, idx = blockIdx.x * 32 + lane;
     const bool live = idx < nw + co, isb = idx >= nw;
     const int tap = isb ? 9 : idx / (co * ci), o = isb ? idx - nw : (idx / ci) % co, i = isb ? 0 : idx % ci;
     const int at[4] = {o * 64 + i, (co + o) * 64 + ci + i, (co + o) * 64 + i, o * 64 + ci + i};
-    double s[4] = {};
+    PairSum ps[4];
     if (live) {
         const float *p = partial + ((size_t)grp * 10 + tap) * 64 * 64;
 #pragma unroll 4
         for (int b = grp; b < nblocks; b += kRedParts, p += (size_t)kRedParts * 10 * 64 * 64) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (!isb || j == 0 || j == 2) s[j] += p[at[j]];
+                if (!isb || j == 0 || j == 2) ps[j].add(p[at[j]]);
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) part[grp][j][lane] = s[j];
+    for (int j = 0; j < 4; ++j) part[grp][j][lane] = make_float2(ps[j].hi, ps[j].lo);
     __syncthreads();
     if (grp == 0 && live) {
+        double s[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            for (int q = 1; q < kRedParts; ++q) s[j] += part[q][j][lane];
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int q = 1; q < kRedParts; ++q) ps[j].add(part[q][j][lane].x, part[q][j][lane].y);
+            s[j] = ps[j].value();
+        }
         float *out = g + (size_t)2 * idx;  // weights [tap][o][i][2], then bias [o][2]
         out[0] = (float)s[0] + (isb ? 0.f : (float)s[1]);
         out[1] = (float)s[2] - (isb ? 0.f : (float)s[3]);
@@ -856,7 +893,7 @@ __global__ void __launch_bounds__(32 * kRedParts)
 // a fixed reference area of 256^2 pixels, so a probe keeps its per-pixel scale
 // whatever the grid it is computed on.
 constexpr double kRefPixels = 65536.0;
-constexpr int kRmsBlocks = 64;  // CTAs an image (one CTA an image: 640 us for 16 of 512^2; now 48)
+constexpr int kRmsBlocks = 64;  // CTAs an image (one CTA an image: 640 us for 16 of 512^2; 48 in FP64 on these, now 16)
 __device__ __forceinline__ double block_sum(double v, double *red) {  // 256 threads, thread 0's result
     red[threadIdx.x] = v;
     __syncthreads();
@@ -869,20 +906,35 @@ __device__ __forceinline__ double block_sum(double v, double *red) {  // 256 thr
 __global__ void __launch_bounds__(256) rms_partial_kernel(const float2 *__restrict__ psi, int HW, double *__restrict__ part) {
     __shared__ double red[256];
     const int b = blockIdx.y;
-    double acc = 0.0;
+    PairSum acc;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < HW; i += gridDim.x * 256) {
         const float2 v = psi[(size_t)b * HW + i];
-        acc += (double)v.x * v.x + (double)v.y * v.y;
+        acc.add_square(v.x);
+        acc.add_square(v.y);
     }
-    const double sum = block_sum(acc, red);
+    double sum = block_sum(acc.value(), red);
+    // squares outside FP32's comfortable range (waves beyond 1e15 or all below 1e-12): in FP64
+    __shared__ bool wide;
+    if (threadIdx.x == 0) wide = !(sum > 1e-24 && sum < 1e30);
+    __syncthreads();
+    if (wide) {
+        double d = 0.0;
+        for (int i = blockIdx.x * 256 + threadIdx.x; i < HW; i += gridDim.x * 256) {
+            const float2 v = psi[(size_t)b * HW + i];
+            d += (double)v.x * v.x + (double)v.y * v.y;
+        }
+        sum = block_sum(d, red);
+    }
     if (threadIdx.x == 0) part[(size_t)b * gridDim.x + blockIdx.x] = sum;
 }
-__global__ void rms_finish_kernel(const double *__restrict__ part, int n, int B, float *__restrict__ s,
-                                  float *__restrict__ inv) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    double r = 0.0;
-    for (int i = 0; i < n; ++i) r += part[(size_t)b * n + i];
+// A warp an image.
+__global__ void rms_finish_kernel(const double *__restrict__ part, float *__restrict__ s, float *__restrict__ inv) {
+    const int b = blockIdx.x, lane = threadIdx.x;
+    static_assert(kRmsBlocks == 64, "two partial sums a lane");
+    double r = part[(size_t)b * kRmsBlocks + lane] + part[(size_t)b * kRmsBlocks + 32 + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+    if (lane) return;
     r = sqrt(r / kRefPixels);
     if (!(r > 0)) r = 1.0;
     s[b] = (float)r;
@@ -1021,7 +1073,7 @@ cudaError_t ClosureNet::forward(const float2 *psi, int B, int H, int W, float2 *
     if ((e = expand(s, nsm, launches)) != cudaSuccess) return e;
     float *sc = scale, *inv = scale + B;
     rms_partial_kernel<<<dim3(kRmsBlocks, B), 256, 0, s>>>(psi, H * W, rms_part);
-    rms_finish_kernel<<<(B + 127) / 128, 128, 0, s>>>(rms_part, kRmsBlocks, B, sc, inv);
+    rms_finish_kernel<<<B, 32, 0, s>>>(rms_part, sc, inv);
     *launches += 2;
     unsigned char *a = (unsigned char *)acts;
     const size_t act = act_bytes(B, H, W);
@@ -1078,9 +1130,9 @@ cudaError_t ClosureNet::backward(int B, int H, int W, int *err, cudaStream_t s, 
         dw_reduce_kernel<<<(9 * co * ci + co + 31) / 32, 32 * kRedParts, 0, s>>>(partial, nblk, co, ci, grads + param_offset(l));
         *launches += 2;
     };
-    const long runs = (long)B * H * (W / 32) / kEdgeWarps;
+    const size_t runs = npix / (32 * kEdgeWarps);
     const int edge_ctas = 2 * nsm < kDwCtas ? 2 * nsm : kDwCtas;
-    const int edge = runs < edge_ctas ? (runs > 0 ? (int)runs : 1) : edge_ctas;
+    const int edge = runs < (size_t)edge_ctas ? (runs > 0 ? (int)runs : 1) : edge_ctas;
     auto wgrad = [&](int l, const __nv_bfloat16 *dy) -> cudaError_t {
         static KernelSetup ks;
         int per_sm = 0;

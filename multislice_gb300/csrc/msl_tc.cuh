@@ -138,5 +138,17 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
     for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Zeros to 64 consecutive columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_zero64(uint32_t taddr) {
+#pragma unroll
+    for (int q = 0; q < 64; q += 16)
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+            "%1};" ::"r"(taddr + (uint32_t)q),
+            "r"(0u)
+            : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 }  // namespace tc
 }  // namespace msl
