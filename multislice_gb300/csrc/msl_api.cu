@@ -945,18 +945,19 @@ int msl_ctem_image(msl_ctx *c, const msl_grid *g, const msl_optics *o, const flo
 
 namespace {
 
-// Host half of a potential build: the atoms validated and binned by slice
-// (stably, so the sum order inside a slice is the input order), the
+// Host half of a potential build: the atoms validated, each given its slice and its rank
+// in it (the input order, so the sum order inside a slice is the input order), and the
 // per-species parameters, laid out as one upload image
-// off | ic | jc | fx | fy | Z | sp | xf | yf | rows | zslot; the device appends the
-// radial tables made from the species' FPARAMS rows.  Each atom is given as its
-// nearest pixel (ic, jc) and the residue x - ic dxp, y - jc dyp formed in FP64 and
-// rounded to float.
+// off | x | y | Z | slice | rank | sp | rows | zslot.  The device sorts the atoms by slice,
+// each as its nearest pixel (ic, jc) and the residue x - ic dxp, y - jc dyp formed in
+// FP64 and rounded to float, and appends the radial tables made from the species'
+// FPARAMS rows.
 struct PotImage {
     std::vector<unsigned char> h;
-    size_t o_off = 0, o_ic = 0, o_jc = 0, o_fx = 0, o_fy = 0, o_z = 0, o_sp = 0, o_xf = 0, o_yf = 0, o_rows = 0, o_tab = 0,
-           o_zs = 0;
-    size_t bytes = 0;  // with the tables, after h
+    size_t o_off = 0, o_x = 0, o_y = 0, o_z = 0, o_k = 0, o_rank = 0, o_sp = 0, o_rows = 0, o_zs = 0;
+    size_t o_ic = 0, o_jc = 0, o_fx = 0, o_fy = 0, o_zd = 0, o_xf = 0, o_yf = 0, o_tab = 0;  // on the device only
+    size_t bytes = 0;  // of all of it
+    int natom = 0;
     int nsp = 0;
     double tab_r0 = 0.15;
 };
@@ -971,7 +972,20 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
     if (at->natom < 0 || (at->natom > 0 && (!at->x || !at->y || !at->z || !at->Z)))
         return fail(c, MSL_E_ARG, "atom arrays are required");
     const double dz = at->cz / nslice;
-    std::vector<int> kz(at->natom), count(nslice + 1, 0);
+    auto up16 = [](size_t x) { return ((x + 15) / 16) * 16; };
+    const size_t na = (size_t)at->natom;
+    im.natom = at->natom;
+    im.o_off = 0;
+    im.o_x = up16(sizeof(int) * (nslice + 1));
+    im.o_y = im.o_x + up16(sizeof(double) * na);
+    im.o_z = im.o_y + up16(sizeof(double) * na);
+    im.o_k = im.o_z + up16(sizeof(int) * na);
+    im.o_rank = im.o_k + up16(sizeof(int) * na);
+    im.o_sp = im.o_rank + up16(sizeof(int) * na);
+    im.o_rows = im.o_sp + up16(sizeof(float) * 104 * 12);
+    im.h.resize(im.o_rows);  // every byte that is read is written below
+    int *kz = (int *)(im.h.data() + im.o_k), *rank = (int *)(im.h.data() + im.o_rank);
+    std::vector<int> count(nslice + 1, 0);
     bool used[104] = {false};
     for (int i = 0; i < at->natom; ++i) {
         if (!is_fin(at->x[i]) || !is_fin(at->y[i]) || !is_fin(at->z[i]))
@@ -981,14 +995,14 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
         if (k >= 0 && (at->Z[i] < 1 || at->Z[i] > 103))
             return fail(c, MSL_E_ARG, "atomic number out of range 1..103 (atom " + std::to_string(i) + ")");
         kz[i] = k;
+        rank[i] = 0;
         if (k >= 0) {
-            count[k + 1]++;
+            rank[i] = count[k + 1]++;
             used[at->Z[i]] = true;
         }
     }
     for (int k = 0; k < nslice; ++k) count[k + 1] += count[k];
-    const int nkeep = count[nslice];
-    const size_t nk = nkeep > 0 ? (size_t)nkeep : 1;
+    const size_t nk = (size_t)count[nslice];  // atoms inside the slices
     // per-species float parameters: A = AL a, B = 2 pi sqrt(b), C = AG c / d, D = pi^2 / d
     // (constants of slicelib.cpp:2673-2674)
     const double AL = 300.8242834, AG = 150.4121417, PIK = 3.141592654;
@@ -1015,55 +1029,43 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
             zlist.push_back(z);
         }
     im.nsp = (zlist.size() <= (size_t)msl::kPotMaxSp && radius > 2 * im.tab_r0) ? (int)zlist.size() : 0;
-    auto up16 = [](size_t x) { return ((x + 15) / 16) * 16; };
-    im.o_off = 0;
-    im.o_ic = up16(sizeof(int) * (nslice + 1));
-    im.o_jc = up16(im.o_ic + sizeof(int) * nk);
-    im.o_fx = up16(im.o_jc + sizeof(int) * nk);
-    im.o_fy = up16(im.o_fx + sizeof(float) * nk);
-    im.o_z = up16(im.o_fy + sizeof(float) * nk);
-    im.o_sp = up16(im.o_z + sizeof(int) * nk);
-    im.o_xf = up16(im.o_sp + sizeof(float) * sp.size());
-    im.o_yf = up16(im.o_xf + sizeof(float) * nk);
-    im.o_rows = up16(im.o_yf + sizeof(float) * nk);
     im.o_zs = im.o_rows + sizeof(double) * 12 * im.nsp;
-    im.o_tab = up16(im.o_zs + sizeof(int) * zslot.size());
-    im.h.assign(im.o_tab, 0);
-    im.bytes = im.o_tab + sizeof(float4) * im.nsp * msl::kPotTabN;
+    im.h.resize(up16(im.o_zs + sizeof(int) * zslot.size()));
     unsigned char *h = im.h.data();
-    int *ics = (int *)(h + im.o_ic), *jcs = (int *)(h + im.o_jc), *zs = (int *)(h + im.o_z);
-    float *fxs = (float *)(h + im.o_fx), *fys = (float *)(h + im.o_fy);
-    float *xf = (float *)(h + im.o_xf), *yf = (float *)(h + im.o_yf);
-    const double dxp = g->ax / g->nx, dyp = g->by / g->ny;
-    std::vector<int> fill(count.begin(), count.end() - 1);
-    for (int i = 0; i < at->natom; ++i) {
-        if (kz[i] < 0) continue;
-        const int p = fill[kz[i]]++;
-        const double xw = at->x[i] - g->ax * std::floor(at->x[i] / g->ax);
-        const double yw = at->y[i] - g->by * std::floor(at->y[i] / g->by);
-        // nearest pixel and the FP64 residue (the same expression as |x - ix dxp|
-        // at that pixel); the pixel index is then wrapped into the grid
-        const double ci = std::floor(xw / dxp + 0.5), cj = std::floor(yw / dyp + 0.5);
-        fxs[p] = (float)(xw - ci * dxp);
-        fys[p] = (float)(yw - cj * dyp);
-        ics[p] = (int)ci % g->nx;
-        jcs[p] = (int)cj % g->ny;
-        zs[p] = at->Z[i];
-        xf[p] = (float)xw;
-        yf[p] = (float)yw;
-    }
     memcpy(h + im.o_off, count.data(), sizeof(int) * (nslice + 1));
+    if (na) {
+        memcpy(h + im.o_x, at->x, sizeof(double) * na);
+        memcpy(h + im.o_y, at->y, sizeof(double) * na);
+        memcpy(h + im.o_z, at->Z, sizeof(int) * na);
+    }
     memcpy(h + im.o_sp, sp.data(), sizeof(float) * sp.size());
     for (int i = 0; i < im.nsp; ++i)
         memcpy(h + im.o_rows + sizeof(double) * 12 * i, fparams + zlist[i] * 12, sizeof(double) * 12);
     memcpy(h + im.o_zs, zslot.data(), sizeof(int) * zslot.size());
+    size_t o = im.h.size();
+    for (size_t *part : {&im.o_ic, &im.o_jc, &im.o_fx, &im.o_fy, &im.o_zd, &im.o_xf, &im.o_yf}) {
+        *part = o;
+        o += up16(sizeof(int) * std::max<size_t>(nk, 1));
+    }
+    im.o_tab = o;
+    im.bytes = o + sizeof(float4) * im.nsp * msl::kPotTabN;
     return MSL_OK;
 }
 
-// Device half: the radial tables, then the gather, on the upload image at `d` (device
-// memory of im.bytes).
+// Device half: the atoms sorted, the radial tables, then the gather, on the upload image
+// at `d` (device memory of im.bytes).
 int potential_launch(msl_ctx *c, const PotImage &im, unsigned char *d, const msl_grid *g, int nslice,
                      double radius, float *vd) {
+    const double dxp = g->ax / g->nx, dyp = g->by / g->ny;
+    LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] {
+                   msl::AtomSort q = {im.natom, (const double *)(d + im.o_x), (const double *)(d + im.o_y),
+                                      (const int *)(d + im.o_z), (const int *)(d + im.o_k),
+                                      (const int *)(d + im.o_rank), (const int *)(d + im.o_off), g->ax, g->by, dxp,
+                                      dyp, g->nx, g->ny, (int *)(d + im.o_ic), (int *)(d + im.o_jc),
+                                      (int *)(d + im.o_zd), (float *)(d + im.o_fx), (float *)(d + im.o_fy),
+                                      (float *)(d + im.o_xf), (float *)(d + im.o_yf)};
+                   return msl::launch_atom_sort(q, c->stream, &c->launches);
+               }));
     // the table reaches 2e-6 beyond the cutoff, so no pixel inside rounds past its end
     const double h = (radius * (1.0 + 2e-6) - im.tab_r0) / msl::kPotTabN;
     if (im.nsp)
@@ -1078,15 +1080,15 @@ int potential_launch(msl_ctx *c, const PotImage &im, unsigned char *d, const msl
     a.fy = (const float *)(d + im.o_fy);
     a.xf = (const float *)(d + im.o_xf);
     a.yf = (const float *)(d + im.o_yf);
-    a.Z = (const int *)(d + im.o_z);
+    a.Z = (const int *)(d + im.o_zd);
     a.off = (const int *)(d + im.o_off);
     a.nslice = nslice;
     a.nx = g->nx;
     a.ny = g->ny;
     a.ax = g->ax;
     a.by = g->by;
-    a.dxp = g->ax / g->nx;
-    a.dyp = g->by / g->ny;
+    a.dxp = dxp;
+    a.dyp = dyp;
     a.dxpf = (float)a.dxp;
     a.dypf = (float)a.dyp;
     a.rad2 = (float)(radius * radius);

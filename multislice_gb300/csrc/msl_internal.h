@@ -144,6 +144,18 @@ struct PotArgs {
 };
 constexpr int kPotTabN = 512;   // cubic pieces per species
 constexpr int kPotMaxSp = 8;    // species the tabulated kernel takes (more: analytic kernel)
+// Atoms into slice order: atom i of slice k[i] (negative: dropped) goes to off[k] + rank[i]
+// as its nearest pixel, residue and float position (PotArgs).
+struct AtomSort {
+    int natom;
+    const double *x, *y;
+    const int *Z, *k, *rank, *off;
+    double ax, by, dxp, dyp;
+    int nx, ny;
+    int *ic, *jc, *zd;
+    float *fx, *fy, *xf, *yf;
+};
+cudaError_t launch_atom_sort(const AtomSort &a, cudaStream_t s, int64_t *launches);
 // Cubic pieces of vzatom (FP64) of width h from r0 for the species whose FPARAMS rows
 // are rows[nsp][12] (device): out[nsp][kPotTabN], in t = -1/2..1/2 about each middle.
 cudaError_t launch_potential_tables(const double *rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,

@@ -261,6 +261,34 @@ cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches
     return cudaGetLastError();
 }
 
+// ------------------------------------------------------------- atoms by slice
+// (97 us on one host core for the 32,000 atoms of the SrTiO3 crystal)
+namespace {
+__global__ void atom_sort_kernel(AtomSort a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.natom || a.k[i] < 0) return;
+    const int p = a.off[a.k[i]] + a.rank[i];
+    const double xw = a.x[i] - a.ax * floor(a.x[i] / a.ax), yw = a.y[i] - a.by * floor(a.y[i] / a.by);
+    // nearest pixel and the FP64 residue (the same expression as |x - ix dxp| at that
+    // pixel); the pixel index is then wrapped into the grid
+    const double ci = floor(xw / a.dxp + 0.5), cj = floor(yw / a.dyp + 0.5);
+    a.fx[p] = (float)(xw - ci * a.dxp);
+    a.fy[p] = (float)(yw - cj * a.dyp);
+    a.ic[p] = (int)ci % a.nx;
+    a.jc[p] = (int)cj % a.ny;
+    a.zd[p] = a.Z[i];
+    a.xf[p] = (float)xw;
+    a.yf[p] = (float)yw;
+}
+}  // namespace
+
+cudaError_t launch_atom_sort(const AtomSort &a, cudaStream_t s, int64_t *launches) {
+    if (a.natom < 1) return cudaSuccess;
+    ++*launches;
+    atom_sort_kernel<<<(a.natom + 127) / 128, 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------ radial tables
 // Cubic pieces of vzatom evaluated in FP64 (slicelib.cpp:2666-2716 with the A&S Bessel
 // polynomials of :168-235), kPotTabN of width h from r0 per species: the cubic through
