@@ -2393,6 +2393,7 @@ struct ExitScan {
     uint8_t *mask = nullptr;
     double *fxy = nullptr, *partial = nullptr;
     int B = 0, ntile = 0, ntrans = 0;
+    bool own_waves = true;  // w: the context's buffer (else set per batch by the caller)
 };
 
 int exit_scan_setup(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float *trans, int ntrans,
@@ -2441,9 +2442,9 @@ int exit_scan_setup(msl_ctx *c, const msl_grid *g, const msl_optics *o, const fl
     if ((size_t)B > max_b) B = (int)max_b;
     if (B > nprobe) B = nprobe;
     X.B = B;
-    CUDA_TRY(c, c->wave.ensure(sizeof(float2) * n2 * B));
+    if (X.own_waves) CUDA_TRY(c, c->wave.ensure(sizeof(float2) * n2 * B));
     CUDA_TRY(c, c->exy.ensure(sizeof(float2) * (size_t)B * (nx + ny) + sizeof(double) * 2 * B));
-    X.w = (float2 *)c->wave.p;
+    X.w = X.own_waves ? (float2 *)c->wave.p : nullptr;
     X.ex = (float2 *)c->exy.p;
     X.ey = X.ex + (size_t)B * nx;
     X.fxy = (double *)(X.ey + (size_t)B * ny);
@@ -2519,13 +2520,17 @@ int msl_stem_exit_waves(msl_ctx *c, const msl_grid *g, const msl_optics *o, cons
     CUDA_TRY(c, cudaSetDevice(c->device));
     if ((rc = err_reset(c))) return rc;
     ExitScan X;
+    // a device output that the passes can take (16-byte aligned) is where the waves live
+    X.own_waves = !(on_device(psi_out) && ((uintptr_t)psi_out & 15u) == 0);
     if ((rc = exit_scan_setup(c, g, o, trans, ntrans, dz, pr, nullptr, nprobe, (size_t)nprobe, X))) return rc;
     const size_t n2 = (size_t)g->nx * g->ny;
     for (int p0 = 0; p0 < nprobe; p0 += X.B) {
         const int nb = std::min(X.B, nprobe - p0);
+        if (!X.own_waves) X.w = (float2 *)psi_out + n2 * p0;
         if ((rc = exit_scan_batch(c, g, X, layer_seq, nslice, probe_xy, p0, nb))) return rc;
-        CUDA_TRY(c, cudaMemcpyAsync(psi_out + 2 * n2 * p0, X.w, sizeof(float2) * n2 * nb, cudaMemcpyDefault,
-                                    c->stream));
+        if (X.own_waves)
+            CUDA_TRY(c, cudaMemcpyAsync(psi_out + 2 * n2 * p0, X.w, sizeof(float2) * n2 * nb, cudaMemcpyDefault,
+                                        c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     }
     collect_profile(c);

@@ -85,7 +85,7 @@ template <> struct ColPlan<384> : ColPlanMixed384 {};
 template <> struct ColPlan<512> : ColPlanT<512, 32, 4, 3, 4> {};
 template <> struct ColPlan<768> : ColPlanMixed768 {};
 template <> struct ColPlan<1024> : ColPlanT<1024, 64, 8, 4, 1> {};
-template <> struct ColPlan<2048> : ColPlanT<2048, 128, 4, 4, 1> {};
+template <> struct ColPlan<2048> : ColPlanT<2048, 128, 4, 4, 1, 2> {};  // two 64 KB tiles: 1 % over three
 
 template <class P> __host__ __device__ constexpr int plan_span(int s) {
     int ns = 1;
