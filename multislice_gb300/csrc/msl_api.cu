@@ -1113,12 +1113,19 @@ namespace {
 int transmission_enqueue(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float *vd, int nlayer,
                          float2 *td, const SliceTables &st, float2 *twr, float2 *twc) {
     const size_t n2 = (size_t)g->nx * g->ny;
-    const double phase_scale = msl_sigma(o->kev) / 1000.0;  // rad per V*A
-    LAUNCH_TRY(c, timed(c, MSL_PROF_OTHER, [&] {
-                   return msl::launch_transmission_phase(vd, phase_scale, n2 * nlayer, td, c->nsm, c->stream,
-                                                         &c->launches);
-               }));
+    const double phase_scale = msl_sigma(o->kev) / 1000.0 / 3.14159265358979323846;  // half turns per V*A
     RowArgs r = row_args(g, twr, nullptr, td, nlayer, msl::ROW_LOAD | msl::ROW_FWD, c->dflag);
+    if (msl::row_gent_side(g->ny, vd, td)) {
+        r.flags = msl::ROW_GENT | msl::ROW_FWD;
+        r.vpot = vd;
+        r.sigma_hi = (float)phase_scale;
+        r.sigma_lo = (float)(phase_scale - (double)r.sigma_hi);
+    } else {
+        LAUNCH_TRY(c, timed(c, MSL_PROF_OTHER, [&] {
+                       return msl::launch_transmission_phase(vd, phase_scale, n2 * nlayer, td, c->nsm, c->stream,
+                                                             &c->launches);
+                   }));
+    }
     LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(g->ny, r, c->stream, c->nsm, &c->launches); }));
     ColArgs ca = col_args(g, st, twc, 0, td, nlayer,
                           msl::COL_LOAD | msl::COL_FWD | msl::COL_PROP | msl::COL_INV | msl::COL_STORE, c->dflag);

@@ -51,7 +51,7 @@ struct KernelSetup {
 // Row pass: contiguous lines of length ny (one line = one ix of one image).
 enum RowFlags {
     ROW_LOAD = 1,    // load the line from `in` (else start from constant 1 + 0i)
-    ROW_GENT = 2,    // start from exp(i * phase_scale * vpot) (FP64 phase)
+    ROW_GENT = 2,    // start from exp(i sigma vpot) (row_gent_side)
     ROW_INV = 4,     // exp(-i) line transform
     ROW_TRANS = 8,   // multiply by trans[ix][iy]
     ROW_FWD = 16,    // exp(+i) line transform
@@ -66,7 +66,7 @@ struct RowArgs {
     int nx;             // lines per image
     const float2 *trans;   // [nx][ny] of the current layer (ROW_TRANS)
     const float *vpot;     // [nx][ny] per image (ROW_GENT)
-    double phase_scale;    // rad per unit of vpot (ROW_GENT)
+    float sigma_hi, sigma_lo;  // half turns per unit of vpot, a sum of two floats (ROW_GENT)
     const float2 *tw;      // twiddle tables of the ny plan
     int flags;
     float scale;           // multiplies the output when != 1
@@ -201,6 +201,7 @@ bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, con
                        const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle);
 
 // Each launcher returns cudaSuccess or the launch error; *launches is bumped.
+bool row_gent_side(int ny, const float *vpot, const float2 *out);
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches);

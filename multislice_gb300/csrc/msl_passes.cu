@@ -90,6 +90,21 @@ __device__ __forceinline__ int spread_id(int w, int n, bool shared) {
     return shared ? (int)blockIdx.x * n + w : w * (int)gridDim.x + (int)blockIdx.x;
 }
 
+// Transmission function exp(i sigma V) of a pixel (mulslice.cpp:414-421), sigma given in
+// half turns as s_hi + s_lo.  The phase carries FP64-grade accuracy in float-float
+// arithmetic (FP64 instructions run at a small fraction of the FP32 rate on this GPU):
+// the product s_hi V is kept exactly as p + e (fma), whole turns are taken off p
+// exactly, the low parts added last, and the remainder in [-1, 1] half turns goes to
+// the single-precision sincospi, which needs no reduction of its own.
+__device__ __forceinline__ float2 phase_grating(float x, float s_hi, float s_lo) {
+    const float p = s_hi * x;
+    const float e = fmaf(s_hi, x, -p) + s_lo * x;  // sigma x = p + e to about 48 bits
+    const float k = 2.0f * rintf(0.5f * p);
+    float sn, cn;
+    sincospif((p - k) + e, &sn, &cn);
+    return make_float2(cn, sn);
+}
+
 // One image's share of a row's running sums; acc: this thread's first element.
 template <int T, int E>
 __device__ __forceinline__ void add_image(double (&sum)[E], const float2 (&v)[E], const RowArgs &a, int img, double *acc) {
@@ -137,18 +152,6 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) row_pass_kernel(RowArgs a)
         if (valid && (a.flags & ROW_LOAD)) {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = a.in[base + t + T * e];
-        } else if (valid && (a.flags & ROW_GENT)) {
-            // t = exp(i sigma V): phase in FP64, reduced to [-pi, pi] before the
-            // single-precision sincos (mulslice.cpp:414-421 forms it in float).
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const double ph = a.phase_scale * (double)a.vpot[base + t + T * e];
-                const double k = rint(ph * 0.15915494309189533577);
-                const double r = fma(-k, 6.283185307179586477, ph);
-                float s, c;
-                sincosf((float)r, &s, &c);
-                v[e] = make_float2(c, s);
-            }
         } else {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = make_float2(valid ? 1.f : 0.f, 0.f);
@@ -1134,7 +1137,9 @@ template <class P_> struct RowTwoCfg {
     static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * W * NBUF + ALIGN;
 };
 
-template <class P>
+// GENT: the lines are transmission functions formed here from the projected potential
+// (4 bytes a pixel in, no elementwise pass before): the first of the band limit's passes.
+template <class P, bool GENT>
 __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row_two_kernel(RowArgs a) {
     using Cfg = RowTwoCfg<P>;
     constexpr int N = Cfg::N, E = P::E, T = P::T, NBUF = Cfg::NBUF, W = Cfg::W, LPW = Cfg::LPW, R0 = Cfg::R0;
@@ -1156,7 +1161,7 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
         mbar_fence_init();
     }
     __syncthreads();  // the only CTA barrier: tables and barriers are ready
-    const bool load = (a.flags & ROW_LOAD) != 0, store = !(a.flags & ROW_NOSTORE);
+    const bool load = GENT || (a.flags & ROW_LOAD) != 0, store = !(a.flags & ROW_NOSTORE);
     const int npairs = a.nlines / LPW;  // units of LPW consecutive lines
     const int G = gridDim.x * W, gw = spread_id(warp, W, a.shared);
     const int nmine = gw < npairs ? (npairs - gw + G - 1) / G : 0;
@@ -1165,8 +1170,13 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
     auto issue = [&](int k) {  // lane 0 only
         const int pair = gw + k * G, s = k % NBUF;
         fence_proxy_async();
-        mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::SLOT);
-        bulk_load(ring + (size_t)s * LPW * N, a.in + (size_t)pair * LPW * N, (uint32_t)Cfg::SLOT, &bar[s]);
+        if constexpr (GENT) {
+            mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::SLOT / 2);
+            bulk_load(ring + (size_t)s * LPW * N, a.vpot + (size_t)pair * LPW * N, (uint32_t)Cfg::SLOT / 2, &bar[s]);
+        } else {
+            mbar_arrive_expect_tx(&bar[s], (uint32_t)Cfg::SLOT);
+            bulk_load(ring + (size_t)s * LPW * N, a.in + (size_t)pair * LPW * N, (uint32_t)Cfg::SLOT, &bar[s]);
+        }
         issued = k + 1;
     };
     if (load && lane == 0 && nmine > 0) issue(0);
@@ -1192,8 +1202,14 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
                 ok = false;
                 break;
             }
+            if constexpr (GENT) {
+                const float *pot = reinterpret_cast<const float *>(slot) + h * N;
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = buf[t + T * e];
+                for (int e = 0; e < E; ++e) v[e] = phase_grating(pot[t + T * e], a.sigma_hi, a.sigma_lo);
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) v[e] = buf[t + T * e];
+            }
         } else {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = make_float2(1.f, 0.f);
@@ -1333,18 +1349,18 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
     }
 }
 
-template <class P> static cudaError_t row_two_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
+template <class P, bool GENT> static cudaError_t row_two_launch_v(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowTwoCfg<P>;
     static KernelSetup ks;
     int per_sm = 0;
     {
-        cudaError_t e = ks.get(row_two_kernel<P>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
+        cudaError_t e = ks.get(row_two_kernel<P, GENT>, Cfg::THREADS, Cfg::SMEM, false, &per_sm);
         if (e != cudaSuccess) return e;
     }
     const int units = spread_units(a.nlines / Cfg::LPW, Cfg::W, a.shared);
     int grid = nsm * per_sm < units ? nsm * per_sm : units;
     if (grid < 1) grid = 1;
-    return launch_pass(row_two_kernel<P>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
+    return launch_pass(row_two_kernel<P, GENT>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, a);
 }
 template <class P> static cudaError_t row_images_launch(const RowArgs &a, cudaStream_t s, int nsm) {
     using Cfg = RowTwoCfg<P>;
@@ -1613,30 +1629,12 @@ __global__ void tilt_wave_kernel(int nx, int ny, const float *xpos, const float 
     out[((size_t)b * nx + ix) * ny + iy] = make_float2((float)cn, (float)sn);
 }
 
-// Transmission function t = exp(i sigma V) of every pixel (mulslice.cpp:414-421).
-// The phase carries FP64-grade accuracy in float-float arithmetic (FP64
-// instructions run at a small fraction of the FP32 rate on this GPU and bound
-// an FP64 version of this elementwise kernel): sigma = s_hi + s_lo, the product
-// s_hi V kept exactly as p + e (fma), then a Cody-Waite reduction by 2 pi split
-// into three floats (C1 = 6.28125 has 8 significant bits, so k C1 is exact for
-// |k| < 2^16), the low parts added last.  The reduced phase in [-pi, pi] then
-// goes to the single-precision sincos.  Elementwise, so the band-limiting
-// transforms that follow run on the fast row / column kernels.
+// t = exp(i sigma V) elementwise, for the sides whose row pass does not form it itself
+// (ROW_GENT).
 __global__ void transmission_phase_kernel(const float *__restrict__ v, float s_hi, float s_lo, size_t n,
                                           float2 *__restrict__ t) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float x = v[i];
-        const float p = s_hi * x;
-        const float e = fmaf(s_hi, x, -p) + s_lo * x;  // sigma x = p + e to about 48 bits
-        const float k = rintf(p * 0.15915494309189535f);
-        float r = fmaf(-k, 6.28125f, p);
-        r = fmaf(-k, 1.9353071693331003e-3f, r);
-        r += e;
-        r = fmaf(-k, 1.0253131677018246e-11f, r);
-        float sn, cn;
-        sincosf(r, &sn, &cn);
-        t[i] = make_float2(cn, sn);
-    }
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        t[i] = phase_grating(v[i], s_hi, s_lo);
 }
 
 // Self-test of the bounded waits: an mbarrier that nothing ever arrives on is
@@ -1836,7 +1834,6 @@ template <int N> static cudaError_t col_tma_launch(const ColArgs &a, cudaStream_
 static bool row_tma_eligible(const RowArgs &a) {
     if (!a.out || ((uintptr_t)a.out & 15u)) return false;
     if ((a.flags & ROW_LOAD) && a.in != a.out) return false;
-    if (a.flags & ROW_GENT) return false;
     return encode_fn() != nullptr;
 }
 
@@ -1877,7 +1874,6 @@ template <int N> static cudaError_t row_tma_launch(const RowArgs &a, cudaStream_
 // Sides whose rows the fast family streams line by line (bulk copies want 16 bytes).
 static bool row_fast_eligible(int ny, const RowArgs &a) {
     if (ny != 256 && ny != 384 && ny != 512 && ny != 768 && ny != 1024 && ny != 2048) return false;
-    if (a.flags & ROW_GENT) return false;
     if (((uintptr_t)a.out & 15u) || ((a.flags & ROW_LOAD) && ((uintptr_t)a.in & 15u))) return false;
     return true;
 }
@@ -1924,6 +1920,14 @@ int sched_col(int n) {
     return k < 0 ? FAM_FAST : g_sched_col[current_device()][k].load(std::memory_order_relaxed);
 }
 }  // namespace
+
+// Whether the row pass of side ny forms transmission functions itself: the two-stage
+// plans of the fast family, from a potential that bulk copies can take.
+bool row_gent_side(int ny, const float *vpot, const float2 *out) {
+    const int fam = sched_row(ny);
+    return (fam == FAM_FAST || fam == FAM_TC) && (ny == 256 || ny == 512 || ny == 1024) &&
+           !(((uintptr_t)vpot | (uintptr_t)out) & 15u);
+}
 
 bool set_schedule(int n, int row_family, int col_family) {
     const int k = side_slot(n);
@@ -2117,7 +2121,8 @@ static TcPassArgs tc_col_args(int nx, const ColArgs &a) {
 }
 
 template <class P> static cudaError_t row_two_launch(const RowArgs &a, cudaStream_t s, int nsm) {
-    return a.nimg ? row_images_launch<P>(a, s, nsm) : row_two_launch_v<P>(a, s, nsm);
+    if (a.nimg) return row_images_launch<P>(a, s, nsm);
+    return a.flags & ROW_GENT ? row_two_launch_v<P, true>(a, s, nsm) : row_two_launch_v<P, false>(a, s, nsm);
 }
 static cudaError_t row_pair_launch(const RowArgs &a, cudaStream_t s, int nsm) {
     return a.nimg ? row_pair_launch_v<true>(a, s, nsm) : row_pair_launch_v<false>(a, s, nsm);
@@ -2131,6 +2136,7 @@ cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, i
     if (fam0 == FAM_TC && row_tc_eligible(ny, a)) return launch_tc_pass(tc_row_args(ny, a), s, nsm, launches);
     ++*launches;
     const int fam = fam0 == FAM_TC ? FAM_FAST : fam0;
+    if ((a.flags & ROW_GENT) && !row_gent_side(ny, a.vpot, a.out)) return cudaErrorInvalidValue;
     if (fam == FAM_FAST && row_fast_eligible(ny, a)) {
         switch (ny) {
             // an image has an even number of rows, so lines always pair up

@@ -28,3 +28,22 @@ def test_potential_paths_match_oracle(ctx, fparams, nx, ny, radius, nz):
     ref = O.potential(x, y, z, spec.Z, fparams, ax, by, cz, nx, ny, ns, radius)
     assert v.shape == ref.shape and np.isfinite(v).all()
     assert O.rel_l2(v, ref) < 1e-5
+
+
+# rows that form the transmission function themselves (256, 512, 1024) and those that
+# start from the elementwise kernel; many turns of phase, both signs; a potential that
+# bulk copies cannot take
+@pytest.mark.parametrize("nx,ny,shift", [(64, 128, 0), (64, 256, 0), (128, 512, 0), (64, 1024, 0), (64, 384, 0),
+                                         (64, 256, 1), (64, 2048, 0)])
+def test_transmission_paths_match_oracle(ctx, nx, ny, shift):
+    import torch
+    rng = np.random.default_rng(nx + ny)
+    ax, by, kev = 9.0, 11.0, 200.0
+    v = rng.uniform(-40000.0, 40000.0, (2, nx, ny)).astype(np.float32)
+    flat = torch.empty(v.size + 4, dtype=torch.float32, device="cuda")
+    dev = flat[shift:shift + v.size].view(2, nx, ny)
+    dev.copy_(torch.from_numpy(v))
+    torch.cuda.synchronize()
+    t = ctx.transmission(dev, ax, by, kev)
+    ref = O.transmission(v.astype(np.float64), kev, ax, by, np.complex128)
+    assert O.rel_l2(t, ref) < 1e-5
