@@ -48,6 +48,7 @@ namespace {
 constexpr int TX = 64, TY = 32, THREADS = 256, PX = TX * TY / THREADS, CAP = 64;
 static_assert(TX == 64 && TY == 32 && THREADS == 256 && PX == 8, "a warp covers 32 x 8 pixels in blocks of 4 x 8");
 constexpr int KR = 2, ROUND = KR * THREADS, NW = THREADS / 32;  // atoms culled per thread per round
+static_assert(KR * NW <= 32, "one warp scans the counts");
 
 __device__ __forceinline__ float poly(const float *c, int n, float t) {
     float s = c[n - 1];
@@ -158,19 +159,20 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
             for (int k = 0; k < KR; ++k) wcount[k * NW + warp] = __popc(ball[k]);
         }
         __syncthreads();
-        // order-preserving positions: atom order is (k, warp, lane)
-        int pos[KR], total = 0;
+        // order-preserving positions: atom order is (k, warp, lane); lane q < KR NW scans
+        // the counts of the (k, warp) pairs in that order
+        int scan = lane < KR * NW ? wcount[lane] : 0;
 #pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            int before = 0, sum = 0;
-            for (int w = 0; w < NW; ++w) {
-                const int n = wcount[k * NW + w];
-                if (w < warp) before += n;
-                sum += n;
-            }
-            pos[k] = total + before + __popc(ball[k] & ((1u << lane) - 1u));
-            total += sum;
+        for (int o = 1; o < KR * NW; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, scan, o);
+            if (lane >= o) scan += up;
         }
+        const int total = __shfl_sync(0xffffffffu, scan, KR * NW - 1);
+        int pos[KR];
+#pragma unroll
+        for (int k = 0; k < KR; ++k)
+            pos[k] = __shfl_sync(0xffffffffu, scan, k * NW + warp) - __popc(ball[k]) +
+                     __popc(ball[k] & ((1u << lane) - 1u));
         for (int piece = 0; piece < total; piece += CAP) {
             if (piece > 0) __syncthreads();  // the previous piece's pair loop is done with the lists
 #pragma unroll
