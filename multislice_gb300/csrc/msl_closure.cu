@@ -427,9 +427,10 @@ __device__ __forceinline__ float2 c_mac(float2 a, float2 w, float2 x) {
 // weight gradient when xin is given.  A warp takes runs of 32 pixels of a row: the
 // 3 x 34 inputs are scaled, rounded to bf16 (as the tensor-core layers see theirs)
 // and kept in shared memory, and each lane holds its channel's weights in registers,
-// so a pixel is 54 operations a lane and its stores are two whole 64-byte halves.  (On the tensor cores the sums round differently, and
-// a flipped bf16 rounding here grows to 5e-4 of the output over the layers.)  16 waves of 512^2: 0.39 ms (2.2 ms with a thread
-// per pixel, whose 64 two-byte stores each touched a line of their own).
+// so a pixel is 54 operations a lane and its stores are two whole 64-byte halves.
+// (On the tensor cores the sums round differently, and a flipped bf16 rounding here
+// grows to 5e-4 of the output over the layers.)  16 waves of 512^2: 0.39 ms (2.2 ms
+// with a thread per pixel, whose 64 two-byte stores each touched a line of their own).
 __global__ void __launch_bounds__(32 * kEdgeWarps, 3)
     first_layer_kernel(const float2 *__restrict__ psi, const float *__restrict__ inv_s, const float *__restrict__ wl,
                        __nv_bfloat162 *__restrict__ xin, __nv_bfloat16 *__restrict__ h, int B, int H, int W) {

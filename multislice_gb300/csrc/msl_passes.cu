@@ -77,6 +77,22 @@ static cudaError_t launch_pass(void (*kern)(KA...), int grid, dim3 block, size_t
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// Column passes overlap only while the waves are small.  Dependents' CTAs land on
+// whatever SM is free, so a tile and its neighbour, which share 128-byte lines, are no
+// longer worked on side by side from pass to pass; once the waves are well past L2 that
+// costs more than the launch gap.  A slice step (row and column pass), columns
+// overlapped / plain:
+//   1024^2:  256 MB 252 / 253 us, 384 MB 368 / 365, 512 MB 503 / 478, 4 GB 5.41 / 4.33 ms
+//    768^2:  288 MB 283 / 285 us, 432 MB 416 / 415, 864 MB 905 / 803
+//    512^2 scan:   2 GB 1.60 / 1.60 ms, 8 GB 6.69 / 6.31;   256^2 and 2048^2, 4 GB: + 1 %
+// At 384 the same is seen from 28 MB on (72 MB 86 / 76 us, 96 MB 106 / 98; 16 MB 25 / 26;
+// 160 MB and more 2 % the other way).  Row passes, whose lines are their own, overlap at
+// any size.
+static bool col_overlaps(const ColArgs &a, int nx) {
+    const size_t limit = (size_t)(nx == 384 ? 20 : 320) << 20;
+    return !a.shared && sizeof(float2) * a.batch * a.ny * nx <= limit;
+}
+
 // CTAs a pass of `units` independent pieces of work is spread over, each CTA able to
 // hold `per_cta` of them at once: one per CTA while the GPU is this pass's alone (a 256^2
 // wave's 32 column tiles on 32 SMs instead of 8), as few CTAs as hold them when other
@@ -1704,7 +1720,7 @@ template <int N> static cudaError_t col_launch(const ColArgs &a, cudaStream_t s,
     int grid = nsm * blocks_per_sm;
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
-    return launch_pass(col_pass_kernel<N>, grid, ColCfg<N>::THREADS, ColCfg<N>::SMEM, s, !a.shared, a);
+    return launch_pass(col_pass_kernel<N>, grid, ColCfg<N>::THREADS, ColCfg<N>::SMEM, s, col_overlaps(a, N), a);
 }
 
 
@@ -1773,7 +1789,7 @@ template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStrea
     if (!col_maps(a, N, Cfg::C, Cfg::BOXR, &map, &mapo)) return cudaErrorInvalidValue;
     const int ntiles = a.batch * (a.ny / Cfg::C);
     const int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
-    return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, mapo, a);
+    return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, col_overlaps(a, N), map, mapo, a);
 }
 
 template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs &a, cudaStream_t s, int nsm) {
@@ -1790,7 +1806,7 @@ template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs 
     const int ntiles = a.batch * (a.ny / Cfg::C);
     int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
     if (grid < 1) grid = 1;
-    return launch_pass(col_tma_kernel<PL, MINB>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, mapo, a);
+    return launch_pass(col_tma_kernel<PL, MINB>, grid, Cfg::THREADS, Cfg::SMEM, s, col_overlaps(a, PL::N), map, mapo, a);
 }
 
 template <class L> static cudaError_t col_half_launch(const ColArgs &a, cudaStream_t s, int nsm) {
@@ -1813,7 +1829,7 @@ template <class L> static cudaError_t col_half_launch(const ColArgs &a, cudaStre
     const int ntiles = spread_units(a.batch * (a.ny / Cfg::C), Cfg::G, a.shared);
     int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
     if (grid < 1) grid = 1;
-    return launch_pass(col_half_kernel<L>, grid, Cfg::THREADS, Cfg::SMEM, s, !a.shared, map, a);
+    return launch_pass(col_half_kernel<L>, grid, Cfg::THREADS, Cfg::SMEM, s, col_overlaps(a, L::N), map, a);
 }
 // The column pass the slice loop takes at side n (0: col_tma_kernel): every
 // pass that loads the wave and starts with the forward transform, with or

@@ -18,7 +18,7 @@
 // culling only has to be conservative) and compacted in atom order (so the
 // float sum order is fixed) into a list of at most 64 atoms at a time.  Each
 // atom arrives as its nearest pixel (ic, jc) and the residue x - ic dxp,
-// y - jc dyp, formed on the host in FP64 and rounded to float, so the offset of
+// y - jc dyp, formed in FP64 (atom_sort_kernel) and rounded to float, so the offset of
 // pixel column ix is |residue + m dxp| with m = ic - ix folded to the minimum
 // image in integers: all in FP32, and an atom sitting exactly on a pixel keeps
 // the FP64 residue there (r is then clamped to 1e-10 A as the reference does,
