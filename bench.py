@@ -677,7 +677,8 @@ def run_potential(args):
     """--potential: the projected potential of one Au 2048^2 configuration (fcc Au
     16x16x40 cells, 80 slices, 3 A cutoff; the frozen-phonon workload's
     per-configuration build) through msl_potential_build into device memory:
-    device time per launch (CUDA events on the library stream) and the pair
+    device time per configuration (CUDA events on the library stream, over the
+    launches of one build) and the pair
     evaluations it makes (pixel-atom pairs inside the cutoff)."""
     import ctypes
 
@@ -701,9 +702,9 @@ def run_potential(args):
     pairs_per_pixel = np.pi * radius ** 2 * spec.natom / nslice / (spec.ax * spec.by)
     pairs = pairs_per_pixel * n * n * nslice
     line = {"workload": "Au fcc 16x16x40 (40,960 atoms, jittered 0.085 A), 2048^2, 80 slices, 3 A cutoff",
-            "ms_per_launch": ms.value / max(k.value, 1), "launches": k.value,
+            "ms_per_configuration": ms.value / reps, "launches": k.value,
             "pixel_size_A": dxp, "pairs_inside_cutoff": pairs,
-            "pairs_per_s": pairs / (ms.value / max(k.value, 1) * 1e-3)}
+            "pairs_per_s": pairs / (ms.value / reps * 1e-3)}
     print(json.dumps(line), flush=True)
 
 

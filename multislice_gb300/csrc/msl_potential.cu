@@ -33,7 +33,7 @@
 // 16-byte table gathers (shared-memory wavefronts at 78 % of peak) and issue (76 %):
 // SrTiO3, 100 slices of 512^2, 5 A cutoff: 0.50 ms (0.69 with warps of 32 rows x 1
 // column, converted piece numbers and a branch per pixel); Au 2048^2, 40 slices, 3 A:
-// 1.10 ms (1.42).
+// 1.08 ms (1.42).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
