@@ -581,7 +581,11 @@ __global__ void __launch_bounds__(ColHalfCfg<L>::THREADS, 1)
     const uint32_t gslot = slot0 + (uint32_t)(g * NBUF) * SLOT;
     const bool store = (a.flags & COL_STORE) != 0;
     const int tpi = a.ny / C, ntiles = a.batch * tpi;
-    const int NG = gridDim.x * G, gid = spread_id(g, G, a.shared);
+    // 256^2 waves past 1 GB (4096 probes, 100 slices: 139.3 ms against 140.5): a CTA's groups on
+    // neighbouring tiles, which share 128-byte lines.  Below that, and at 512 and 1024,
+    // neighbours on different SMs are as fast or faster (512, 256 waves: 207 us against 211).
+    const bool dense = N == 256 && a.batch * (a.ny / C) >= 65536;
+    const int NG = gridDim.x * G, gid = spread_id(g, G, a.shared || dense);
     const int nmine = gid < ntiles ? (ntiles - gid + NG - 1) / NG : 0;
     pass_begin();
     int issued = 0;

@@ -1,5 +1,6 @@
 """Column passes launched as programmatic dependents up to a size of the waves and
-plainly above it: each wave of a batch on either side of the line equals its own run."""
+plainly above it, and 256^2 tiles dealt differently past 65536 of them: each wave of a
+batch on either side of a line equals its own run."""
 import numpy as np
 import pytest
 
@@ -7,7 +8,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,batch", [(384, 17), (384, 18), (768, 71), (768, 72), (1024, 40), (1024, 41)])
+@pytest.mark.parametrize("n,batch", [(256, 2047), (256, 2048), (384, 17), (384, 18), (768, 71), (768, 72), (1024, 40), (1024, 41)])
 def test_batches_on_both_sides_of_the_overlap_limit(n, batch):
     from multislice_gb300 import Context
 
