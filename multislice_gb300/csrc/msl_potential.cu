@@ -63,7 +63,10 @@ __constant__ float kK0B[7] = {1.25331414f, -0.07832358f, 0.02189568f, -0.0106244
                               -0.00251540f, 0.00053208f};
 
 constexpr float kRound = 12582912.0f;  // 1.5 2^23: adding it rounds to an integer
-// 1 / sqrt(x) of x > 0, denormals taken as 0.
+// Least |dy| of a pair, so that r^2 is never 0 or a denormal (whose reciprocal root
+// below is infinite): far below the 1e-10 A at which r is clamped.
+constexpr float kTiny = 1.2e-19f;
+// 1 / sqrt(x) of a normal x > 0 (denormals are taken as 0).
 __device__ __forceinline__ float rsqrt_normal(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
                 int m = sjc[k] - (iy0 + i);
                 if (2 * m >= a.ny) m -= a.ny;
                 else if (2 * m < -a.ny) m += a.ny;
-                sdy[k][i] = fabsf(fmaf((float)m, a.dypf, sfy[k]));
+                sdy[k][i] = fmaxf(fabsf(fmaf((float)m, a.dypf, sfy[k])), kTiny);
             }
             __syncthreads();
             for (int k = 0; k < n; ++k) {
@@ -224,8 +227,7 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
                     if (TAB) {
                         // cubic piece of the tabulated profile in t = u - i, |t| <= 1/2, about the
                         // middle of the piece i nearest u: rounded by adding 1.5 2^23, so that no
-                        // pair takes a conversion (a pixel beyond the cutoff lands on any piece;
-                        // r = 0 gives a NaN and takes the analytic form)
+                        // pair takes a conversion (a pixel beyond the cutoff lands on any piece)
                         const float u = fmaf(r2 * rsqrt_normal(r2), a.tab_inv_h, a.tab_off);
                         const float m = u + kRound;
                         const float t = u - (m - kRound);
