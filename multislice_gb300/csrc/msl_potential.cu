@@ -115,13 +115,15 @@ __global__ void __launch_bounds__(THREADS, 4) potential_kernel(PotArgs a) {
     const int txs = 8 * (4 * (warp >> 2) + (lane >> 3));
     const int iy0 = blockIdx.x * TY, ix0 = blockIdx.y * TX, s = blockIdx.z;
 
-    // tile bounding box (pixel positions) for the culling, in float with a margin
-    // that covers the float rounding of the coordinates (the culling only has to
-    // keep every atom that can reach the tile; the pair loop tests r < radius)
+    // tile bounding box (pixel positions) for the culling, in float.  The culling only has
+    // to keep every atom that can reach the tile (the pair loop tests r < radius), so the
+    // margin covers the rounding of the positions at any cell size: the atom's, the tile
+    // middle's (pixel size and product), the cell edge's and two differences, each at most
+    // 2^-24 of the cell edge, 3.6e-7 of it together.
     const float xc = ((float)ix0 + 0.5f * (TX - 1)) * a.dxpf, hx = 0.5f * (TX - 1) * a.dxpf;
     const float yc = ((float)iy0 + 0.5f * (TY - 1)) * a.dypf, hy = 0.5f * (TY - 1) * a.dypf;
     const float axf = (float)a.ax, byf = (float)a.by;
-    const float rad = sqrtf(a.rad2) * (1.0f + 1e-5f) + 1e-3f;
+    const float rad = sqrtf(a.rad2) * (1.0f + 1e-5f) + 1e-3f + 4e-7f * fmaxf(axf, byf);
     const int a0 = a.off[s], a1 = a.off[s + 1];
     float acc[PX];
 #pragma unroll

@@ -1,5 +1,6 @@
 """The potential gather at the ends of its number range: atoms a denormal squared
-distance from a pixel -- against the FP64 oracle."""
+distance from a pixel, and cells so large that float positions are coarse against the
+culling's margin -- against the FP64 oracle."""
 import numpy as np
 import pytest
 
@@ -25,4 +26,25 @@ def test_atoms_a_hair_from_a_pixel(ctx, fparams, extra):
     v = ctx.potential(S.Specimen(x, y, z, Z, ax, by, float(ns)), n, n, ns, radius)
     ref = O.potential(x, y, z, Z, fparams, ax, by, float(ns), n, n, ns, radius)
     assert np.isfinite(v).all()
+    assert O.rel_l2(v, ref) < 1e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(2048, 64), (64, 2048)])
+def test_atoms_just_inside_the_cutoff_of_a_tile_in_a_large_cell(ctx, fparams, nx, ny):
+    """Each atom reaches one pixel only, the last or first of a 64 x 32-pixel tile, from
+    0.1 mA inside the cutoff; at 20 um a float position is off by up to 1 mA."""
+    px, radius, ns = 9.77, 1.0, 1
+    ax, by = nx * px, ny * px
+    dx, dy = ax / nx, by / ny
+    t = np.arange(0, 2048, 64 if nx == 2048 else 32)
+    near = radius - 1e-4
+    along = np.concatenate([(t + (63 if nx == 2048 else 31)) * (dx if nx == 2048 else dy) + near,
+                            np.maximum(t * (dx if nx == 2048 else dy) - near, 0.0)[1:]])
+    across = (np.arange(len(along)) % 61 + 1) * (dy if nx == 2048 else dx)
+    x, y = (along, across) if nx == 2048 else (across, along)
+    z = np.full(len(x), 0.5)
+    Z = np.full(len(x), 79, np.int32)
+    v = ctx.potential(S.Specimen(x, y, z, Z, ax, by, 1.0), nx, ny, ns, radius)
+    ref = O.potential(x, y, z, Z, fparams, ax, by, 1.0, nx, ny, ns, radius)
+    assert np.count_nonzero(ref) >= len(x)
     assert O.rel_l2(v, ref) < 1e-5
