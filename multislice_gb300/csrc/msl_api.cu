@@ -2539,10 +2539,15 @@ int msl_stem_exit_waves(msl_ctx *c, const msl_grid *g, const msl_optics *o, cons
     CUDA_TRY(c, cudaSetDevice(c->device));
     if ((rc = err_reset(c))) return rc;
     ExitScan X;
-    // a device output that the passes can take (16-byte aligned) is where the waves live
-    X.own_waves = !(on_device(psi_out) && ((uintptr_t)psi_out & 15u) == 0);
-    if ((rc = exit_scan_setup(c, g, o, trans, ntrans, dz, pr, nullptr, nprobe, (size_t)nprobe, X))) return rc;
     const size_t n2 = (size_t)g->nx * g->ny;
+    // a device output that the passes can take is where the waves live
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, psi_out) == cudaSuccess)
+        X.own_waves = !msl::loop_runs_in(at, c->device, psi_out, sizeof(float2) * n2 * nprobe, trans,
+                                         sizeof(float2) * n2 * ntrans);
+    else
+        cudaGetLastError();
+    if ((rc = exit_scan_setup(c, g, o, trans, ntrans, dz, pr, nullptr, nprobe, (size_t)nprobe, X))) return rc;
     for (int p0 = 0; p0 < nprobe; p0 += X.B) {
         const int nb = std::min(X.B, nprobe - p0);
         if (!X.own_waves) X.w = (float2 *)psi_out + n2 * p0;

@@ -200,6 +200,17 @@ void prop_tables(int nx, int ny, const msl_optics *o, double dz, const float *kx
 bool encode_tensor_map(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const uint64_t *dims,
                        const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle);
 
+// Whether a slice loop may run in a caller's buffer instead of the context's own: memory
+// of the context's GPU (not another GPU's, which its kernels may not reach, nor managed
+// memory, which may be elsewhere), aligned for the passes' bulk copies, and apart from
+// what the loop reads.
+inline bool loop_runs_in(const cudaPointerAttributes &at, int device, const void *p, size_t bytes, const void *read,
+                         size_t read_bytes) {
+    const uintptr_t a = (uintptr_t)p, r = (uintptr_t)read;
+    return at.type == cudaMemoryTypeDevice && at.device == device && (a & 15u) == 0 &&
+           (a + bytes <= r || r + read_bytes <= a);
+}
+
 // Each launcher returns cudaSuccess or the launch error; *launches is bumped.
 bool row_gent_side(int ny, const float *vpot, const float2 *out);
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches);
