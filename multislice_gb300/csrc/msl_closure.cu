@@ -906,9 +906,10 @@ __device__ __forceinline__ double block_sum(double v, double *red) {  // 256 thr
 }
 __global__ void __launch_bounds__(256) rms_partial_kernel(const float2 *__restrict__ psi, int HW, double *__restrict__ part) {
     __shared__ double red[256];
-    const int b = blockIdx.y;
+    // images and their blocks both on x, which takes any number of images
+    const int b = blockIdx.x / kRmsBlocks, q = blockIdx.x % kRmsBlocks;
     PairSum acc;
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < HW; i += gridDim.x * 256) {
+    for (int i = q * 256 + threadIdx.x; i < HW; i += kRmsBlocks * 256) {
         const float2 v = psi[(size_t)b * HW + i];
         acc.add_square(v.x);
         acc.add_square(v.y);
@@ -920,13 +921,13 @@ __global__ void __launch_bounds__(256) rms_partial_kernel(const float2 *__restri
     __syncthreads();
     if (wide) {
         double d = 0.0;
-        for (int i = blockIdx.x * 256 + threadIdx.x; i < HW; i += gridDim.x * 256) {
+        for (int i = q * 256 + threadIdx.x; i < HW; i += kRmsBlocks * 256) {
             const float2 v = psi[(size_t)b * HW + i];
             d += (double)v.x * v.x + (double)v.y * v.y;
         }
         sum = block_sum(d, red);
     }
-    if (threadIdx.x == 0) part[(size_t)b * gridDim.x + blockIdx.x] = sum;
+    if (threadIdx.x == 0) part[blockIdx.x] = sum;
 }
 // A warp an image.
 __global__ void rms_finish_kernel(const double *__restrict__ part, float *__restrict__ s, float *__restrict__ inv) {
@@ -1073,7 +1074,7 @@ cudaError_t ClosureNet::forward(const float2 *psi, int B, int H, int W, float2 *
     if (e != cudaSuccess) return e;
     if ((e = expand(s, nsm, launches)) != cudaSuccess) return e;
     float *sc = scale, *inv = scale + B;
-    rms_partial_kernel<<<dim3(kRmsBlocks, B), 256, 0, s>>>(psi, H * W, rms_part);
+    rms_partial_kernel<<<kRmsBlocks * B, 256, 0, s>>>(psi, H * W, rms_part);
     rms_finish_kernel<<<B, 32, 0, s>>>(rms_part, sc, inv);
     *launches += 2;
     unsigned char *a = (unsigned char *)acts;
