@@ -62,21 +62,24 @@ inline int param_offset(int l) {
 inline int param_count() { return param_offset(kLayers); }
 
 // ------------------------------------------------------------------ helpers
-// A running sum as an unevaluated pair hi + lo (Knuth's two-sum, 48 bits): FP64 adds
-// and conversions run at a few per clock and SM here and bounded the reductions.
-struct PairSum {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float x, float tail = 0.f) {
-        const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)), tail));
-        hi = s;
+// A running sum as three unevaluated floats, two error-free additions (Knuth's two-sum)
+// and a plain one for what is left: some 72 bits, more than an FP64 sum keeps, at 13
+// FP32 additions a value.  FP64 ones run at a few per clock and SM here.
+struct TripleSum {
+    float hi = 0.f, mid = 0.f, lo = 0.f;
+    __device__ __forceinline__ static float two_sum(float &a, float x) {  // a <- a + x, the error returned
+        const float s = __fadd_rn(a, x), b = __fsub_rn(s, a);
+        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, b)), __fsub_rn(x, b));
+        a = s;
+        return e;
     }
-    __device__ __forceinline__ void add_square(float x) {
-        const float p = __fmul_rn(x, x);
-        add(p, fmaf(x, x, -p));
+    __device__ __forceinline__ void add(float x) {
+        float e = two_sum(hi, x);
+        e = two_sum(mid, e);
+        lo = __fadd_rn(lo, e);
     }
-    // (an infinite or overflowed sum has a NaN tail)
-    __device__ __forceinline__ double value() const { return isfinite(lo) ? (double)hi + (double)lo : (double)hi; }
+    // NaN where a sum on the way overflowed (or a value was no number)
+    __device__ __forceinline__ double value() const { return ((double)lo + (double)mid) + (double)hi; }
 };
 __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
 
@@ -854,16 +857,16 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
 // the sum of its two Wr blocks and dWi the difference of the others; db likewise.
 // 32 parameters a block, their partials shared among kRedParts threads each (one
 // thread over all of them waited for its loads: 105 us for 152 CTAs; FP64 sums took
-// 29, float pairs 17).
+// 33, three-float ones 19).
 constexpr int kRedParts = 16;
 __global__ void __launch_bounds__(32 * kRedParts)
     dw_reduce_kernel(const float *__restrict__ partial, int nblocks, int co, int ci, float *__restrict__ g) {
-    __shared__ float2 part[kRedParts][4][32];
+    __shared__ float part[kRedParts][4][3][32];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, nw = 9 * co * ci, idx = blockIdx.x * 32 + lane;
     const bool live = idx < nw + co, isb = idx >= nw;
     const int tap = isb ? 9 : idx / (co * ci), o = isb ? idx - nw : (idx / ci) % co, i = isb ? 0 : idx % ci;
     const int at[4] = {o * 64 + i, (co + o) * 64 + ci + i, (co + o) * 64 + i, o * 64 + ci + i};
-    PairSum ps[4];
+    TripleSum ps[4];
     if (live) {
         const float *p = partial + ((size_t)grp * 10 + tap) * 64 * 64;
 #pragma unroll 4
@@ -874,15 +877,25 @@ __global__ void __launch_bounds__(32 * kRedParts)
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) part[grp][j][lane] = make_float2(ps[j].hi, ps[j].lo);
+    for (int j = 0; j < 4; ++j) {
+        part[grp][j][0][lane] = ps[j].hi;
+        part[grp][j][1][lane] = ps[j].mid;
+        part[grp][j][2][lane] = ps[j].lo;
+    }
     __syncthreads();
     if (grp == 0 && live) {
         double s[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
 #pragma unroll
-            for (int q = 1; q < kRedParts; ++q) ps[j].add(part[q][j][lane].x, part[q][j][lane].y);
+            for (int q = 1; q < kRedParts; ++q)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ps[j].add(part[q][j][i][lane]);
             s[j] = ps[j].value();
+            if (!isfinite(s[j])) {  // beyond float's range on the way: FP64 has room
+                s[j] = 0.0;
+                for (int b = 0; b < nblocks; ++b) s[j] += partial[((size_t)b * 10 + tap) * 64 * 64 + at[j]];
+            }
         }
         float *out = g + (size_t)2 * idx;  // weights [tap][o][i][2], then bias [o][2]
         out[0] = (float)s[0] + (isb ? 0.f : (float)s[1]);
@@ -894,7 +907,7 @@ __global__ void __launch_bounds__(32 * kRedParts)
 // a fixed reference area of 256^2 pixels, so a probe keeps its per-pixel scale
 // whatever the grid it is computed on.
 constexpr double kRefPixels = 65536.0;
-constexpr int kRmsBlocks = 64;  // CTAs an image (one CTA an image: 640 us for 16 of 512^2; 48 in FP64 on these, now 16)
+constexpr int kRmsBlocks = 64;  // CTAs an image (one CTA an image: 640 us for 16 of 512^2, now 48, of FP64 operations)
 __device__ __forceinline__ double block_sum(double v, double *red) {  // 256 threads, thread 0's result
     red[threadIdx.x] = v;
     __syncthreads();
@@ -908,25 +921,12 @@ __global__ void __launch_bounds__(256) rms_partial_kernel(const float2 *__restri
     __shared__ double red[256];
     // images and their blocks both on x, which takes any number of images
     const int b = blockIdx.x / kRmsBlocks, q = blockIdx.x % kRmsBlocks;
-    PairSum acc;
+    double acc = 0.0;
     for (int i = q * 256 + threadIdx.x; i < HW; i += kRmsBlocks * 256) {
         const float2 v = psi[(size_t)b * HW + i];
-        acc.add_square(v.x);
-        acc.add_square(v.y);
+        acc += (double)v.x * v.x + (double)v.y * v.y;
     }
-    double sum = block_sum(acc.value(), red);
-    // squares outside FP32's comfortable range (waves beyond 1e15 or all below 1e-12): in FP64
-    __shared__ bool wide;
-    if (threadIdx.x == 0) wide = !(sum > 1e-24 && sum < 1e30);
-    __syncthreads();
-    if (wide) {
-        double d = 0.0;
-        for (int i = q * 256 + threadIdx.x; i < HW; i += kRmsBlocks * 256) {
-            const float2 v = psi[(size_t)b * HW + i];
-            d += (double)v.x * v.x + (double)v.y * v.y;
-        }
-        sum = block_sum(d, red);
-    }
+    const double sum = block_sum(acc, red);
     if (threadIdx.x == 0) part[blockIdx.x] = sum;
 }
 // A warp an image.
