@@ -157,7 +157,7 @@ enum Epi { EPI_BIAS_RELU = 0, EPI_MASK = 1 };
 constexpr size_t kWTile = 64 * 128;          // one tap's B tile: 64 rows x 128 bytes
 constexpr size_t kATile = kTile * 128;       // 128 pixels x 128 bytes
 constexpr int kRing = 7, kStage = 2, kAcc = 8;
-constexpr int kDwThreads = 192;                    // TMA warp, MMA warp, four that read the sums out
+constexpr int kDwThreads = 320;                    // TMA warp, MMA warp, eight that read the sums out
 constexpr int kConvThreads = 64 + 128 * kStage;    // TMA warp, MMA warp, a four-warp epilogue group per staging tile
 constexpr size_t kConvSmem = 1024 + 9 * kWTile + (kRing + kStage) * kATile;
 
@@ -646,7 +646,14 @@ __global__ void __launch_bounds__(32 * kEdgeWarps, 3)
 // dW[tap][n][k] = sum_p dy[p][n] x[p + tap][k] and db[n] = sum_p dy[p][n].  Every
 // CTA writes FP32 sums over its own pixels, partial[cta][10][n][k] (row 9: the
 // bias, k = 0); dw_reduce_kernel adds them in CTA order.
-constexpr int kDwCtas = 320;                 // most CTAs of a weight-gradient launch
+// A CTA's float sums run over kDwChain pixels at most, whatever the batch (their error
+// grows with their length): an edge layer's lane over half of them, then over the warps;
+// on the tensor cores in pieces of kDwRows rows, because adding into tensor memory
+// truncates, which on 16384 pixels of random waves is off by 1.9e-5 where rounded sums
+// are by 2.4e-6 (2.8e-6 in pieces).  Batches of more than that many pixels an SM (2.4 M in
+// all) take more CTAs than SMs.
+constexpr int kDwChain = 16384;
+constexpr int kDwRows = 16;  // of 128 pixels
 constexpr size_t kDwStage = 6 * kATile;      // three x rows, dy at three column shifts
 constexpr size_t kDwSmem = 1024 + 2 * kDwStage + 2048;
 
@@ -662,16 +669,18 @@ __device__ __forceinline__ uint64_t desc_pixel_major(uint32_t addr, uint32_t lbo
 // by each column tap, and per 16 pixels two MMAs of M = 128, N = 192 add every tap
 // at once: A is x rows (y - 1, y), then (y + 1, a tile of ones for the bias sum), B
 // the three shifted dy tiles.  The two accumulators (128 x 192) stay in tensor
-// memory over all rows of the CTA.  bf16 products are exact in FP32.  Bound by the
-// stages' 96 KB per 128 pixels from L2 beside 16 x 96 MMA cycles.
-// 8 waves of 256^2 (64 x 64 channels): 5.7 ms on the CUDA cores, now 40 us.
+// memory for kDwRows rows, after which eight warps add them, rounded, to the CTA's
+// partial sums.  bf16 products are exact in FP32.  Bound by the stages' 96 KB per 128
+// pixels from L2 beside 16 x 96 MMA cycles.
+// 8 waves of 256^2 (64 x 64 channels): 5.7 ms on the CUDA cores, now 49 us (40 with one
+// read-out at the end, 112 with four warps that fetch a sum when they add to it).
 __global__ void __launch_bounds__(kDwThreads, 1)
     dw_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mdy, Units units,
                  float *__restrict__ partial, int *err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *ones = base + 2 * kDwStage;   // 16 pixels x 64 channels of 1
-    __shared__ uint64_t full[2], empty[2], done;
+    __shared__ uint64_t full[2], empty[2], done, read, last;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform
@@ -683,6 +692,8 @@ __global__ void __launch_bounds__(kDwThreads, 1)
             mbar_init(&empty[i], 1);
         }
         mbar_init(&done, 1);
+        mbar_init(&read, 8);
+        mbar_init(&last, 1);
         mbar_fence_init();
         failed = 0;
     }
@@ -724,6 +735,8 @@ __global__ void __launch_bounds__(kDwThreads, 1)
             for (int y = y0; y < y1; ++y, ++n) {
                 const uint32_t s = n & 1u;
                 if (!(ok = wait_or_quit(&full[s], (n / 2) & 1, &failed))) break;
+                const uint32_t f = n / kDwRows, r = n % kDwRows;
+                if (r == 0 && f > 0 && !(ok = wait_or_quit(&read, (f - 1) & 1, &failed))) break;
                 tc::fence_after_sync();
                 if (tc::elect_one()) {
                     const uint32_t st = sb + s * (uint32_t)kDwStage;
@@ -731,42 +744,80 @@ __global__ void __launch_bounds__(kDwThreads, 1)
                     for (int k = 0; k < kTile / 16; ++k) {
                         const uint32_t x = st + k * 2048u, x2 = x + 2u * (uint32_t)kATile;
                         const uint64_t bd = desc_pixel_major(x + 3u * (uint32_t)kATile, (uint32_t)kATile);
-                        const uint32_t acc = (n > 0 || k > 0) ? 1u : 0u;
+                        const uint32_t acc = (r > 0 || k > 0) ? 1u : 0u;
                         tc::mma_bf16(tmem, desc_pixel_major(x, (uint32_t)kATile), bd, idesc, acc);
                         tc::mma_bf16(tmem + 256u, desc_pixel_major(x2, so - x2), bd, idesc, acc);
                     }
                     tc::mma_commit(&empty[s]);
+                    if (r == kDwRows - 1) tc::mma_commit(&done);
                 }
                 __syncwarp();
             }
         }
-        if (tc::elect_one()) tc::mma_commit(&done);
-        if (!mbar_wait_bounded(&done, 0, kWait)) failed = 1;
+        if (tc::elect_one()) {
+            if (ok && n % kDwRows) tc::mma_commit(&done);
+            tc::mma_commit(&last);  // every MMA has completed before the CTA's memory goes
+        }
+        if (!mbar_wait_bounded(&last, 0, kWait)) failed = 1;
         __syncwarp();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    if (warp >= 2 && !failed) {
+    } else {
         // lane m of the first accumulator: x channel m % 64 of row tap m / 64, column (column tap, n);
         // of the second: row tap 2, and from m = 64 on the bias sum
         float *p = partial + (size_t)blockIdx.x * 10 * 64 * 64;
         const int m = 32 * (warp & 3) + lane, k = m & 63;
         const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
-        for (int c0 = 0; c0 < 192; c0 += 16) {
-            const int kx = c0 >> 6, n0 = c0 & 63;
-            float v[16], w[16];
-            tc::tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-            tc::tmem_ld16(tmem + 256u + lane_base + (uint32_t)c0, w);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                p[(((m >> 6) * 3 + kx) * 64 + n0 + j) * 64 + k] = v[j];
-                if (m < 64) p[((6 + kx) * 64 + n0 + j) * 64 + k] = w[j];
-                else if (m == 64 && kx == 1) p[(9 * 64 + n0 + j) * 64] = w[j];
-            }
+        int rows = 0;
+        for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+            int b, x0, y0, y1;
+            units.get(u, &b, &x0, &y0, &y1);
+            rows += y1 - y0;
         }
-        tc::fence_before_sync();
+        // a warp reads half the columns, kCols at a time, whose sums so far it fetches ahead
+        constexpr int kCols = 32;
+        const int cbeg = warp < 6 ? 0 : 96, cend = cbeg + 96;
+        float old[2][kCols];
+        auto at = [&](int half, int c) {
+            const int tap = half ? 6 + c / 64 : (m >> 6) * 3 + c / 64;
+            return half && m >= 64 ? (9 * 64 + c % 64) * 64 : (tap * 64 + c % 64) * 64 + k;
+        };
+        auto mine = [&](int half, int c) { return !half || m < 64 || (m == 64 && c / 64 == 1); };
+        auto fetch = [&](int c0) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < kCols; ++j) old[i][j] = mine(i, c0 + j) ? p[at(i, c0 + j)] : 0.f;
+        };
+        for (int f = 0; f * kDwRows < rows; ++f) {
+            if (f) fetch(cbeg);
+            if (__any_sync(0xffffffffu, !wait_or_quit(&done, f & 1, &failed))) break;
+            tc::fence_after_sync();
+#pragma unroll 1
+            for (int c0 = cbeg; c0 < cend; c0 += kCols) {
+                float v[2][kCols];
+#pragma unroll
+                for (int j = 0; j < kCols; j += 16) {
+                    tc::tmem_ld16(tmem + lane_base + (uint32_t)(c0 + j), &v[0][j]);
+                    tc::tmem_ld16(tmem + 256u + lane_base + (uint32_t)(c0 + j), &v[1][j]);
+                }
+                if (f) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < kCols; ++j) v[i][j] = __fadd_rn(old[i][j], v[i][j]);
+                    if (c0 + kCols < cend) fetch(c0 + kCols);  // while these are stored
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < kCols; ++j)
+                        if (mine(i, c0 + j)) p[at(i, c0 + j)] = v[i][j];
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&read);
+        }
     }
+    tc::fence_before_sync();
     __syncthreads();
     if (failed && tid == 0 && err) atomicExch(err, 1);
     if (warp == 1) tc::tmem_free(tmem, 512);
@@ -966,6 +1017,25 @@ inline int grid_for(size_t n, int threads, int nsm) {
     const size_t cap = (size_t)nsm * 8;
     return (int)(g < cap ? (g > 0 ? g : 1) : cap);
 }
+// Strips and CTAs of the tensor-core weight gradients.
+inline Units dw_units(int B, int H, int W, int nsm, int *grid) {
+    Units u = plan_units(B, H, W, nsm, 0);
+    const int rows = kDwChain / kTile, n = u.count();
+    *grid = n < nsm ? n : nsm;
+    if ((n + *grid - 1) / *grid * u.seg > rows) {
+        const int segs = (H + rows - 1) / rows;
+        u.seg = (H + segs - 1) / segs;
+        const int per = rows / u.seg;
+        *grid = (u.count() + per - 1) / per;
+    }
+    return u;
+}
+// CTAs of the edge layers' weight gradients.
+inline int dw_edge_grid(size_t npix, int nsm) {
+    const size_t runs = npix / (32 * kEdgeWarps), most = kDwChain / 64;  // of 32 pixels a warp
+    const size_t ctas = runs < 2 * (size_t)nsm ? (runs > 0 ? runs : 1) : 2 * (size_t)nsm;
+    return (int)(runs > ctas * most ? (runs + most - 1) / most : ctas);
+}
 // CTAs of the kernels with a warp per 32 pixels
 inline int edge_grid(size_t npix, int nsm) { return grid_for(npix, 32 * kEdgeWarps, nsm); }
 }  // namespace
@@ -995,7 +1065,7 @@ void ClosureNet::release() {
     acts = nullptr;
     loss_part = rms_part = nullptr;
     cap_bytes = cap_pix = 0;
-    cap_img = 0;
+    cap_img = cap_part = 0;
 }
 
 // Bytes of one padded activation, and of the workspace of a batch: training keeps
@@ -1003,11 +1073,22 @@ void ClosureNet::release() {
 static size_t act_bytes(int B, int H, int W) { return ((Pad{H, W}.pixels(B) * 128 + 255) / 256) * 256; }
 static size_t plain_bytes(size_t npix, size_t per) { return ((npix * per + 255) / 256) * 256; }
 
-cudaError_t ClosureNet::ensure(int B, int H, int W, bool train) {
+cudaError_t ClosureNet::ensure(int B, int H, int W, bool train, int nsm) {
     const size_t npix = (size_t)B * H * W;
-    const size_t bytes = train ? 7 * act_bytes(B, H, W) + plain_bytes(npix, 4) + plain_bytes(npix, 8)
+    int part = 0;  // CTAs whose weight-gradient sums are kept
+    if (train) {
+        dw_units(B, H, W, nsm, &part);
+        const int e = dw_edge_grid(npix, nsm);
+        part = part > e ? part : e;
+    }
+    size_t bytes = train ? 7 * act_bytes(B, H, W) + plain_bytes(npix, 4) + plain_bytes(npix, 8)
                                : 2 * act_bytes(B, H, W);
-    if (bytes > cap_bytes || npix > cap_pix || B > cap_img || (train && !partial)) {
+    if (bytes > cap_bytes || npix > cap_pix || B > cap_img || part > cap_part) {
+        // every part at least as large as it was, so that two shapes in turn allocate once
+        bytes = bytes > cap_bytes ? bytes : cap_bytes;
+        part = part > cap_part ? part : cap_part;
+        const size_t pix = npix > cap_pix ? npix : cap_pix;
+        const int img = B > cap_img ? B : cap_img;
         if (acts) cudaFree(acts);
         if (partial) cudaFree(partial);
         if (loss_part) cudaFree(loss_part);
@@ -1019,16 +1100,17 @@ cudaError_t ClosureNet::ensure(int B, int H, int W, bool train) {
         scale = nullptr;
         rms_part = nullptr;
         cap_bytes = cap_pix = 0;
-        cap_img = 0;
+        cap_img = cap_part = 0;
         cudaError_t e;
         if ((e = cudaMalloc(&acts, bytes)) != cudaSuccess) return e;
-        if (train && (e = cudaMalloc(&partial, sizeof(float) * kDwCtas * 10 * 64 * 64)) != cudaSuccess) return e;
+        if (part && (e = cudaMalloc(&partial, sizeof(float) * part * 10 * 64 * 64)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&loss_part, sizeof(double) * 4096)) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&scale, sizeof(float) * 2 * B)) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&rms_part, sizeof(double) * kRmsBlocks * B)) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&scale, sizeof(float) * 2 * img)) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&rms_part, sizeof(double) * kRmsBlocks * img)) != cudaSuccess) return e;
         cap_bytes = bytes;
-        cap_pix = npix;
-        cap_img = B;
+        cap_pix = pix;
+        cap_img = img;
+        cap_part = part;
     }
     return cudaSuccess;
 }
@@ -1070,7 +1152,7 @@ cudaError_t ClosureNet::forward(const float2 *psi, int B, int H, int W, float2 *
                                 bool train, int *err, cudaStream_t s, int nsm, int64_t *launches) {
     if (W % kTile || H < 3 || W < 3) return cudaErrorInvalidValue;
     const size_t npix = (size_t)B * H * W;
-    cudaError_t e = ensure(B, H, W, train);
+    cudaError_t e = ensure(B, H, W, train, nsm);
     if (e != cudaSuccess) return e;
     if ((e = expand(s, nsm, launches)) != cudaSuccess) return e;
     float *sc = scale, *inv = scale + B;
@@ -1126,15 +1208,12 @@ cudaError_t ClosureNet::forward(const float2 *psi, int B, int H, int W, float2 *
 cudaError_t ClosureNet::backward(int B, int H, int W, int *err, cudaStream_t s, int nsm, int64_t *launches) {
     const size_t npix = (size_t)B * H * W;
     cudaError_t e;
-    const int ctas = nsm < kDwCtas ? nsm : kDwCtas;
     auto reduce = [&](int l, int nblk) {
         const int co = layer_co(l), ci = layer_ci(l);
         dw_reduce_kernel<<<(9 * co * ci + co + 31) / 32, 32 * kRedParts, 0, s>>>(partial, nblk, co, ci, grads + param_offset(l));
         *launches += 2;
     };
-    const size_t runs = npix / (32 * kEdgeWarps);
-    const int edge_ctas = 2 * nsm < kDwCtas ? 2 * nsm : kDwCtas;
-    const int edge = runs < (size_t)edge_ctas ? (runs > 0 ? (int)runs : 1) : edge_ctas;
+    const int edge = dw_edge_grid(npix, nsm);
     auto wgrad = [&](int l, const __nv_bfloat16 *dy) -> cudaError_t {
         static KernelSetup ks;
         int per_sm = 0;
@@ -1142,8 +1221,8 @@ cudaError_t ClosureNet::backward(int B, int H, int W, int *err, cudaStream_t s, 
         if (e != cudaSuccess) return e;
         CUtensorMap mx, mdy;
         if (!act_map(&mx, hbuf[l], B, H, W, 3) || !act_map(&mdy, dy, B, H, W, 1)) return cudaErrorInvalidValue;
-        const Units u = plan_units(B, H, W, ctas, 0);
-        const int grid = u.count() < ctas ? u.count() : ctas;
+        int grid;
+        const Units u = dw_units(B, H, W, nsm, &grid);
         dw_tc_kernel<<<grid, kDwThreads, kDwSmem, s>>>(mx, mdy, u, partial, err);
         reduce(l, grid);
         return cudaGetLastError();

@@ -320,14 +320,14 @@ struct ClosureNet {
     double *rms_part = nullptr;       // per-block sums of |psi|^2
     float *scale = nullptr;           // per-image s and 1/s
     size_t cap_bytes = 0, cap_pix = 0;
-    int cap_img = 0;
+    int cap_img = 0, cap_part = 0;
     int step = 0;
     int loss_blocks = 0;
     __nv_bfloat16 *hbuf[6] = {}, *dh[2] = {}, *xbuf = nullptr;
     float *g6 = nullptr;
     cudaError_t alloc_params();
     void release();
-    cudaError_t ensure(int B, int H, int W, bool train);
+    cudaError_t ensure(int B, int H, int W, bool train, int nsm);
     cudaError_t expand(cudaStream_t s, int nsm, int64_t *launches);
     cudaError_t conv_tc(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
                         const __nv_bfloat16 *mask, __nv_bfloat16 *out, int B, int H, int W, int epi, int *err,
