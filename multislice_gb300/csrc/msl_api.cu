@@ -311,24 +311,19 @@ int build_slice_tables(msl_ctx *c, const msl_grid *g, const msl_optics *o, int n
     // FP64 phases are turned into tables on the device; the reference's float phases
     // and the identity propagator (band limit and ifft scale only) on the host
     const bool dev = dz && !o->f32_prop_args;
-    const size_t off = dev ? fbytes + sizeof(msl::PropTable) * ntrans : fbytes;  // of the tables
-    CUDA_TRY(c, tb.ensure(off + pbytes));
+    CUDA_TRY(c, tb.ensure(fbytes + pbytes));
     st.d_kx2 = (float *)tb.p;
     st.d_ky2 = st.d_kx2 + nx;
     st.d_kx = st.d_ky2 + ny;
     st.d_ky = st.d_kx + nx;
-    st.d_prop = (float2 *)((unsigned char *)tb.p + off);
-    std::vector<unsigned char> h(dev ? off : off + pbytes);
+    st.d_prop = (float2 *)((unsigned char *)tb.p + fbytes);
+    std::vector<unsigned char> h(dev ? fbytes : fbytes + pbytes);
     memcpy(h.data(), st.kx2.data(), sizeof(float) * nx);
     memcpy(h.data() + sizeof(float) * nx, st.ky2.data(), sizeof(float) * ny);
     memcpy(h.data() + sizeof(float) * (nx + ny), st.kx.data(), sizeof(float) * nx);
     memcpy(h.data() + sizeof(float) * (2 * nx + ny), st.ky.data(), sizeof(float) * ny);
-    if (dev) {
-        msl::PropTable *pt = (msl::PropTable *)(h.data() + fbytes);
-        const double lam = msl_wavelength(o->kev), ttx = 2.0 * tan(o->tilt_x), tty = 2.0 * tan(o->tilt_y);
-        for (int l = 0; l < ntrans; ++l) pt[l] = {st.d_kx, dz[l], lam, ttx, tty};
-    } else {
-        float2 *hp = (float2 *)(h.data() + off);
+    if (!dev) {
+        float2 *hp = (float2 *)(h.data() + fbytes);
         for (int l = 0; l < ntrans; ++l) {
             float2 *px = hp + (size_t)l * (nx + ny), *py = px + nx;
             if (dz) {
@@ -342,9 +337,12 @@ int build_slice_tables(msl_ctx *c, const msl_grid *g, const msl_optics *o, int n
     }
     int rc = upload(c, tb, h.data(), h.size());
     if (rc) return rc;
-    if (dev)
-        CUDA_TRY(c, msl::launch_prop_tables((const msl::PropTable *)((unsigned char *)tb.p + fbytes), ntrans, nx, ny,
-                                            st.d_prop, c->stream));
+    if (dev) {
+        std::vector<msl::PropTable> pt(ntrans);
+        const double lam = msl_wavelength(o->kev), ttx = 2.0 * tan(o->tilt_x), tty = 2.0 * tan(o->tilt_y);
+        for (int l = 0; l < ntrans; ++l) pt[l] = {(float)g->ax, (float)g->by, dz[l], lam, ttx, tty};
+        CUDA_TRY(c, msl::launch_prop_tables(pt.data(), ntrans, nx, ny, st.d_prop, c->stream));
+    }
     return MSL_OK;
 }
 
@@ -1336,7 +1334,8 @@ struct JobGroup {
     int nx = 0, ny = 0;
     std::vector<int> ids;
     size_t wave_off = 0, tab_off = 0, ptab_off = 0, stage_off = 0, apchi_off = 0, exy_off = 0;
-    size_t kbytes = 0, dbytes = 0, nprop = 0, prop_off = 0;  // frequencies, table descriptions, tables
+    size_t kbytes = 0, nprop = 0, prop_off = 0;  // frequencies, propagator tables
+    std::vector<msl::PropTable> prop;
     std::vector<std::vector<size_t>> layer_prop;  // per job, per layer: row of its propagator table
     float2 *twr = nullptr, *twc = nullptr;
 };
@@ -1385,12 +1384,11 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
             }
             if (jb.illumination == MSL_PROBE) probes = true;
         }
-        g.kbytes = align256(sizeof(float) * 2 * (g.nx + g.ny) * nb);  // kx2 ky2 kx ky per job
-        g.dbytes = align256(sizeof(msl::PropTable) * g.nprop);
+        g.kbytes = align256(sizeof(float) * (g.nx + g.ny) * nb);  // kx2 ky2 per job
         g.wave_off = wave_bytes;
         wave_bytes = align256(wave_bytes + sizeof(float2) * n2 * nb);
         g.tab_off = tab_bytes;
-        tab_bytes += g.kbytes + g.dbytes;
+        tab_bytes += g.kbytes;
         g.prop_off = prop_bytes;
         prop_bytes = align256(prop_bytes + sizeof(float2) * (g.nx + g.ny) * g.nprop);
         g.ptab_off = ptab_bytes;
@@ -1413,7 +1411,7 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
     // a column of ones (the plane wave's ky = 0 column) after the tables
     const size_t ones_off = tab_bytes;
     tab_bytes = align256(tab_bytes + sizeof(float2) * 2048);
-    // uploaded: the frequencies, descriptions and the ones; then the propagator tables
+    // uploaded: the frequencies and the ones; then the propagator tables
     CUDA_TRY(c, c->wave.ensure(wave_bytes));
     CUDA_TRY(c, c->tabs.ensure(tab_bytes + prop_bytes));
     CUDA_TRY(c, c->jobtab.ensure(ptab_bytes));
@@ -1444,25 +1442,22 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
                 so = align256(so + bytes);
             }
         }
-        // [kx2 ky2 kx ky] floats per job, then a propagator table's description per distinct thickness
+        // [kx2 ky2] floats per job, a propagator table per distinct thickness
         float *hk2 = (float *)(htab.data() + g.tab_off);
-        msl::PropTable *hprop = (msl::PropTable *)(htab.data() + g.tab_off + g.kbytes);
         const float *dk = (const float *)(dtab + g.tab_off);
+        g.prop.resize(g.nprop);
         std::vector<float> k2max(nb);
         for (int b = 0; b < nb; ++b) {
             const msl_job &jb = jobs[g.ids[b]];
             std::vector<float> kx, kx2, ky, ky2;
             freqn_f32(nx, jb.grid.ax, kx, kx2);
             freqn_f32(ny, jb.grid.by, ky, ky2);
-            float *hk = hk2 + (size_t)b * 2 * (nx + ny);
-            memcpy(hk, kx2.data(), sizeof(float) * nx);
-            memcpy(hk + nx, ky2.data(), sizeof(float) * ny);
-            memcpy(hk + nx + ny, kx.data(), sizeof(float) * nx);
-            memcpy(hk + 2 * nx + ny, ky.data(), sizeof(float) * ny);
+            memcpy(hk2 + (size_t)b * (nx + ny), kx2.data(), sizeof(float) * nx);
+            memcpy(hk2 + (size_t)b * (nx + ny) + nx, ky2.data(), sizeof(float) * ny);
             k2max[b] = k2max_f32(nx, ny, jb.grid.ax, jb.grid.by, bandlimit);
             const double lam = msl_wavelength(jb.kev);
             for (int l = 0; l < jb.ntrans; ++l)
-                hprop[g.layer_prop[b][l]] = {dk + (size_t)b * 2 * (nx + ny) + nx + ny, jb.dz[l], lam, 0.0, 0.0};
+                g.prop[g.layer_prop[b][l]] = {(float)jb.grid.ax, (float)jb.grid.by, jb.dz[l], lam, 0.0, 0.0};
         }
         // pointer tables: trans[S][nb], prop[S][nb], k2[nb], then k2max[nb]
         const float2 *dp = (const float2 *)(dtab + tab_bytes + g.prop_off);
@@ -1474,7 +1469,7 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
                 pt[(size_t)s * nb + b] = tdev[b] + (size_t)l * n2;
                 pt[(size_t)(S + s) * nb + b] = dp + g.layer_prop[b][l] * (nx + ny);
             }
-        for (int b = 0; b < nb; ++b) pt[(size_t)2 * S * nb + b] = dk + (size_t)b * 2 * (nx + ny);
+        for (int b = 0; b < nb; ++b) pt[(size_t)2 * S * nb + b] = dk + (size_t)b * (nx + ny);
         memcpy(pt + (size_t)2 * S * nb + nb, k2max.data(), sizeof(float) * nb);
         // probe k-vectors and positions
         for (int b = 0; b < nb; ++b) {
@@ -1519,7 +1514,7 @@ int run_job_groups(msl_ctx *c, const msl_job *jobs, std::vector<JobGroup> &group
             if (!st) return fail(c, MSL_E_CUDA, "stream creation failed");
             CUDA_TRY(c, cudaStreamWaitEvent(st, fork, 0));
         }
-        CUDA_TRY(c, msl::launch_prop_tables((const msl::PropTable *)(dtab + g.tab_off + g.kbytes), (int)g.nprop, nx, ny,
+        CUDA_TRY(c, msl::launch_prop_tables(g.prop.data(), (int)g.nprop, nx, ny,
                                             (float2 *)(dtab + tab_bytes + g.prop_off), st));
         float2 *w = (float2 *)((unsigned char *)c->wave.p + g.wave_off);
         const unsigned char *tp = dptab + g.ptab_off;

@@ -216,11 +216,12 @@ bool row_gent_side(int ny, const float *vpot, const float2 *out);
 cudaError_t launch_row_pass(int ny, const RowArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, int64_t *launches);
 cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches);
-// One propagator table: float frequencies kx[nx] then ky[ny] (device), slice
-// thickness, wavelength and 2 tan(tilt); out[ntab][nx + ny].  Part of a call's set-up
-// like its uploads: not counted as a launch.
+// One propagator table: cell edges (frequencies as freqn_f32), slice thickness,
+// wavelength and 2 tan(tilt); out[ntab][nx + ny].  The descriptions (host) travel as
+// kernel arguments, so a call needs no scratch for them.  Part of a call's set-up like
+// its uploads: not counted as a launch.
 struct PropTable {
-    const float *k;
+    float ax, by;
     double dz, lam, ttx, tty;
 };
 cudaError_t launch_prop_tables(const PropTable *tabs, int ntab, int nx, int ny, float2 *out, cudaStream_t s);

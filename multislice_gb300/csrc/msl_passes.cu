@@ -1549,16 +1549,22 @@ template <bool IMG> static cudaError_t row_pair_launch_v(const RowArgs &a, cudaS
 // table, py carrying the ifft scale.  On one host core the sines and cosines of a
 // 16-layer 256^2 call took 0.10 ms before its first pass could start, those of 6
 // layers at 2048^2 0.3 ms.
-__global__ void prop_table_kernel(const PropTable *tabs, int nx, int ny, float scale, float2 *out) {
+template <int CAP> struct PropTables {
+    PropTable t[CAP];
+};
+template <int CAP>
+__global__ void prop_table_kernel(const __grid_constant__ PropTables<CAP> tabs, int nx, int ny, float scale, float2 *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx + ny) return;
-    const PropTable p = tabs[blockIdx.y];
-    const double k = (double)p.k[i];
-    const double t = 3.14159265358979323846 * p.dz * (k * k * p.lam - k * (i < nx ? p.ttx : p.tty));
+    const PropTable &p = tabs.t[blockIdx.y];
+    const bool x = i < nx;
+    const int j = x ? i : i - nx, n = x ? nx : ny;
+    const double k = (double)__fdiv_rn((float)(j > n / 2 ? j - n : j), x ? p.ax : p.by);  // freqn_f32
+    const double t = 3.14159265358979323846 * p.dz * (k * k * p.lam - k * (x ? p.ttx : p.tty));
     double sn, cn;
     sincos(t, &sn, &cn);
     const float re = (float)cn, im = (float)-sn;
-    out[(size_t)blockIdx.y * (nx + ny) + i] = i < nx ? make_float2(re, im) : make_float2(re * scale, im * scale);
+    out[(size_t)blockIdx.y * (nx + ny) + i] = x ? make_float2(re, im) : make_float2(re * scale, im * scale);
 }
 
 __global__ void probe_table_kernel(int nx, int ny, const double *kxd, const double *kyd,
@@ -2217,12 +2223,19 @@ cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, i
     }
 }
 
+template <int CAP>
+static void prop_tables_v(const PropTable *tabs, int n, int nx, int ny, float2 *out, cudaStream_t s) {
+    PropTables<CAP> a;
+    memcpy(a.t, tabs, sizeof(PropTable) * n);
+    prop_table_kernel<CAP><<<dim3((nx + ny + 127) / 128, n), 128, 0, s>>>(a, nx, ny, 1.0f / ((float)nx * (float)ny), out);
+}
 cudaError_t launch_prop_tables(const PropTable *tabs, int ntab, int nx, int ny, float2 *out, cudaStream_t s) {
-    const float scale = 1.0f / ((float)nx * (float)ny);
-    for (int t = 0; t < ntab; t += 65535) {  // grid.y limit
-        const int n = ntab - t < 65535 ? ntab - t : 65535;
-        prop_table_kernel<<<dim3((nx + ny + 127) / 128, n), 128, 0, s>>>(tabs + t, nx, ny, scale,
-                                                                        out + (size_t)t * (nx + ny));
+    constexpr int kFew = 32, kMany = 512;  // 1.3 and 20 KB of arguments (of 32)
+    for (int t = 0; t < ntab; t += kMany) {
+        const int n = ntab - t < kMany ? ntab - t : kMany;
+        float2 *o = out + (size_t)t * (nx + ny);
+        if (n <= kFew) prop_tables_v<kFew>(tabs + t, n, nx, ny, o, s);
+        else prop_tables_v<kMany>(tabs + t, n, nx, ny, o, s);
     }
     return cudaGetLastError();
 }
