@@ -11,6 +11,7 @@
 #include <atomic>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -943,21 +944,23 @@ int msl_ctem_image(msl_ctx *c, const msl_grid *g, const msl_optics *o, const flo
 
 namespace {
 
-// Host half of a potential build: the atoms validated, each given its slice and its rank
-// in it (the input order, so the sum order inside a slice is the input order), and the
-// per-species parameters, laid out as one upload image
-// off | x | y | Z | slice | rank | sp | rows | zslot.  The device sorts the atoms by slice,
-// each as its nearest pixel (ic, jc) and the residue x - ic dxp, y - jc dyp formed in
-// FP64 and rounded to float, and appends the radial tables made from the species'
-// FPARAMS rows.
+// Host half of a potential build: the atoms validated, each inside the slices given its
+// slice and its rank in it (the input order, so the sum order inside a slice is the input
+// order), and the per-species parameters, laid out as an upload image off | sp | zslot.
+// The device sorts the atoms by slice, each as its nearest pixel (ic, jc) and the residue
+// x - ic dxp, y - jc dyp formed in FP64 and rounded to float, and makes the radial tables
+// from the species' FPARAMS rows, both behind the image.
 struct PotImage {
     std::vector<unsigned char> h;
-    size_t o_off = 0, o_x = 0, o_y = 0, o_z = 0, o_k = 0, o_rank = 0, o_sp = 0, o_rows = 0, o_zs = 0;
+    std::unique_ptr<msl::AtomIn[]> in;
+    size_t in_cap = 0, nk = 0;  // atoms inside the slices
+    size_t o_off = 0, o_sp = 0, o_zs = 0;
     size_t o_ic = 0, o_jc = 0, o_fx = 0, o_fy = 0, o_zd = 0, o_xf = 0, o_yf = 0, o_tab = 0;  // on the device only
-    size_t bytes = 0;  // of all of it
-    int natom = 0;
+    size_t bytes = 0;  // of all of it on the device
     int nsp = 0;
+    msl::PotRows rows;
     double tab_r0 = 0.15;
+    size_t in_bytes() const { return sizeof(msl::AtomIn) * nk; }
 };
 
 int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, const msl_grid *g, int nslice,
@@ -971,18 +974,11 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
         return fail(c, MSL_E_ARG, "atom arrays are required");
     const double dz = at->cz / nslice;
     auto up16 = [](size_t x) { return ((x + 15) / 16) * 16; };
-    const size_t na = (size_t)at->natom;
-    im.natom = at->natom;
-    im.o_off = 0;
-    im.o_x = up16(sizeof(int) * (nslice + 1));
-    im.o_y = im.o_x + up16(sizeof(double) * na);
-    im.o_z = im.o_y + up16(sizeof(double) * na);
-    im.o_k = im.o_z + up16(sizeof(int) * na);
-    im.o_rank = im.o_k + up16(sizeof(int) * na);
-    im.o_sp = im.o_rank + up16(sizeof(int) * na);
-    im.o_rows = im.o_sp + up16(sizeof(float) * 104 * 12);
-    im.h.resize(im.o_rows);  // every byte that is read is written below
-    int *kz = (int *)(im.h.data() + im.o_k), *rank = (int *)(im.h.data() + im.o_rank);
+    if (im.in_cap < (size_t)at->natom) {
+        im.in.reset(new msl::AtomIn[at->natom]);
+        im.in_cap = at->natom;
+    }
+    size_t nk = 0;
     std::vector<int> count(nslice + 1, 0);
     bool used[104] = {false};
     for (int i = 0; i < at->natom; ++i) {
@@ -992,15 +988,13 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
         if (at->z[i] < 0.0 || k < 0 || k >= nslice) k = -1;
         if (k >= 0 && (at->Z[i] < 1 || at->Z[i] > 103))
             return fail(c, MSL_E_ARG, "atomic number out of range 1..103 (atom " + std::to_string(i) + ")");
-        kz[i] = k;
-        rank[i] = 0;
         if (k >= 0) {
-            rank[i] = count[k + 1]++;
+            im.in[nk++] = {at->x[i], at->y[i], k, count[k + 1]++, at->Z[i]};
             used[at->Z[i]] = true;
         }
     }
+    im.nk = nk;
     for (int k = 0; k < nslice; ++k) count[k + 1] += count[k];
-    const size_t nk = (size_t)count[nslice];  // atoms inside the slices
     // per-species float parameters: A = AL a, B = 2 pi sqrt(b), C = AG c / d, D = pi^2 / d
     // (constants of slicelib.cpp:2673-2674)
     const double AL = 300.8242834, AG = 150.4121417, PIK = 3.141592654;
@@ -1027,19 +1021,15 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
             zlist.push_back(z);
         }
     im.nsp = (zlist.size() <= (size_t)msl::kPotMaxSp && radius > 2 * im.tab_r0) ? (int)zlist.size() : 0;
-    im.o_zs = im.o_rows + sizeof(double) * 12 * im.nsp;
-    im.h.resize(up16(im.o_zs + sizeof(int) * zslot.size()));
+    im.o_off = 0;
+    im.o_sp = up16(sizeof(int) * (nslice + 1));
+    im.o_zs = im.o_sp + sizeof(float) * sp.size();
+    im.h.resize(im.o_zs + sizeof(int) * zslot.size());
     unsigned char *h = im.h.data();
     memcpy(h + im.o_off, count.data(), sizeof(int) * (nslice + 1));
-    if (na) {
-        memcpy(h + im.o_x, at->x, sizeof(double) * na);
-        memcpy(h + im.o_y, at->y, sizeof(double) * na);
-        memcpy(h + im.o_z, at->Z, sizeof(int) * na);
-    }
     memcpy(h + im.o_sp, sp.data(), sizeof(float) * sp.size());
-    for (int i = 0; i < im.nsp; ++i)
-        memcpy(h + im.o_rows + sizeof(double) * 12 * i, fparams + zlist[i] * 12, sizeof(double) * 12);
     memcpy(h + im.o_zs, zslot.data(), sizeof(int) * zslot.size());
+    for (int i = 0; i < im.nsp; ++i) memcpy(im.rows.r[i], fparams + zlist[i] * 12, sizeof(im.rows.r[i]));
     size_t o = im.h.size();
     for (size_t *part : {&im.o_ic, &im.o_jc, &im.o_fx, &im.o_fy, &im.o_zd, &im.o_xf, &im.o_yf}) {
         *part = o;
@@ -1050,25 +1040,33 @@ int potential_prepare(msl_ctx *c, const msl_atoms *at, const double *fparams, co
     return MSL_OK;
 }
 
-// Device half: the atoms sorted, the radial tables, then the gather, on the upload image
-// at `d` (device memory of im.bytes).
-int potential_launch(msl_ctx *c, const PotImage &im, unsigned char *d, const msl_grid *g, int nslice,
-                     double radius, float *vd) {
+// Device half: the image uploaded to `d` (device memory of im.bytes), the atoms sorted,
+// the radial tables, then the gather.  The unsorted atoms pass through the memory of the
+// potential, which the gather fills last (a few hundred at a time at worst), so that the
+// build takes no scratch beyond what the gather reads.  h, in: the image and the atoms,
+// in host memory that stays until the stream has drained.
+int potential_launch(msl_ctx *c, const PotImage &im, const void *h, const msl::AtomIn *in, unsigned char *d,
+                     const msl_grid *g, int nslice, double radius, float *vd) {
     const double dxp = g->ax / g->nx, dyp = g->by / g->ny;
-    LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] {
-                   msl::AtomSort q = {im.natom, (const double *)(d + im.o_x), (const double *)(d + im.o_y),
-                                      (const int *)(d + im.o_z), (const int *)(d + im.o_k),
-                                      (const int *)(d + im.o_rank), (const int *)(d + im.o_off), g->ax, g->by, dxp,
-                                      dyp, g->nx, g->ny, (int *)(d + im.o_ic), (int *)(d + im.o_jc),
-                                      (int *)(d + im.o_zd), (float *)(d + im.o_fx), (float *)(d + im.o_fy),
-                                      (float *)(d + im.o_xf), (float *)(d + im.o_yf)};
-                   return msl::launch_atom_sort(q, c->stream, &c->launches);
-               }));
+    CUDA_TRY(c, cudaMemcpyAsync(d, h, im.h.size(), cudaMemcpyHostToDevice, c->stream));
+    const uintptr_t v0 = (uintptr_t)vd, v1 = v0 + sizeof(float) * (size_t)nslice * g->nx * g->ny, st = (v0 + 15) & ~(uintptr_t)15;
+    const size_t piece = (v1 - st) / sizeof(msl::AtomIn);
+    for (size_t i = 0; i < im.nk; i += piece) {
+        const size_t n = std::min(piece, im.nk - i);
+        CUDA_TRY(c, cudaMemcpyAsync((void *)st, in + i, sizeof(msl::AtomIn) * n, cudaMemcpyHostToDevice, c->stream));
+        LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] {
+                       msl::AtomSort q = {(int)n, (const msl::AtomIn *)st, (const int *)(d + im.o_off), g->ax, g->by,
+                                          dxp, dyp, g->nx, g->ny, (int *)(d + im.o_ic), (int *)(d + im.o_jc),
+                                          (int *)(d + im.o_zd), (float *)(d + im.o_fx), (float *)(d + im.o_fy),
+                                          (float *)(d + im.o_xf), (float *)(d + im.o_yf)};
+                       return msl::launch_atom_sort(q, c->stream, &c->launches);
+                   }));
+    }
     // the table reaches 2e-6 beyond the cutoff, so no pixel inside rounds past its end
-    const double h = (radius * (1.0 + 2e-6) - im.tab_r0) / msl::kPotTabN;
+    const double step = (radius * (1.0 + 2e-6) - im.tab_r0) / msl::kPotTabN;
     if (im.nsp)
         LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] {
-                       return msl::launch_potential_tables((const double *)(d + im.o_rows), im.nsp, im.tab_r0, h,
+                       return msl::launch_potential_tables(im.rows, im.nsp, im.tab_r0, step,
                                                            (float4 *)(d + im.o_tab), c->stream, &c->launches);
                    }));
     msl::PotArgs a;
@@ -1095,8 +1093,8 @@ int potential_launch(msl_ctx *c, const PotImage &im, unsigned char *d, const msl
     a.tab = (const float4 *)(d + im.o_tab);
     a.zslot = (const int *)(d + im.o_zs);
     a.nsp = im.nsp;
-    a.tab_inv_h = (float)(1.0 / h);
-    a.tab_off = (float)(-im.tab_r0 / h - 0.5);
+    a.tab_inv_h = (float)(1.0 / step);
+    a.tab_off = (float)(-im.tab_r0 / step - 0.5);
     LAUNCH_TRY(c, timed(c, MSL_PROF_POTENTIAL, [&] { return msl::launch_potential(a, c->stream, &c->launches); }));
     return MSL_OK;
 }
@@ -1217,7 +1215,7 @@ struct PhononBuilder {
         const int sl = cfg & 1;
         if (prepared[sl] != cfg && (rc = prepare(cfg))) return rc;
         const PotImage &m = im[sl];
-        const size_t bytes = m.h.size(), dbytes = m.bytes;
+        const size_t hbytes = m.h.size(), bytes = hbytes + m.in_bytes(), dbytes = m.bytes;
         if (bytes > pin_cap) {  // (re)allocate both pinned buffers with headroom
             for (int i = 0; i < 2; ++i) {
                 CUDA_TRY(c, cudaEventSynchronize(ev[i]));
@@ -1232,10 +1230,12 @@ struct PhononBuilder {
             CUDA_TRY(c, atoms.ensure(dbytes + dbytes / 4));
         }
         CUDA_TRY(c, cudaEventSynchronize(ev[sl]));  // the upload two configurations back has read pin[sl]
-        memcpy(pin[sl], m.h.data(), bytes);
-        CUDA_TRY(c, cudaMemcpyAsync(atoms.p, pin[sl], bytes, cudaMemcpyHostToDevice, c->stream));
+        memcpy(pin[sl], m.h.data(), hbytes);
+        if (m.nk) memcpy(pin[sl] + hbytes, m.in.get(), m.in_bytes());
+        if ((rc = potential_launch(c, m, pin[sl], (const msl::AtomIn *)(pin[sl] + hbytes), (unsigned char *)atoms.p, g,
+                                   nslice, radius, (float *)pot.p)))
+            return rc;
         CUDA_TRY(c, cudaEventRecord(ev[sl], c->stream));
-        if ((rc = potential_launch(c, m, (unsigned char *)atoms.p, g, nslice, radius, (float *)pot.p))) return rc;
         if ((rc = transmission_enqueue(c, g, o, (const float *)pot.p, nslice, t, st, twr, twc))) return rc;
         if (cfg + 1 < nconfig && (rc = prepare(cfg + 1))) return rc;
         return MSL_OK;
@@ -1902,7 +1902,6 @@ int msl_potential_build(msl_ctx *c, const msl_atoms *at, const double *fparams, 
     if ((rc = potential_prepare(c, at, fparams, g, nslice, radius, im))) return rc;
     CUDA_TRY(c, cudaSetDevice(c->device));
     CUDA_TRY(c, c->atoms.ensure(im.bytes));
-    if ((rc = upload(c, c->atoms, im.h.data(), im.h.size()))) return rc;
     const size_t vbytes = sizeof(float) * (size_t)nslice * g->nx * g->ny;
     float *vd;
     const bool vdev = on_device(v_out);
@@ -1912,7 +1911,8 @@ int msl_potential_build(msl_ctx *c, const msl_atoms *at, const double *fparams, 
         CUDA_TRY(c, c->pot.ensure(vbytes));
         vd = (float *)c->pot.p;
     }
-    if ((rc = potential_launch(c, im, (unsigned char *)c->atoms.p, g, nslice, radius, vd))) return rc;
+    if ((rc = potential_launch(c, im, im.h.data(), im.in.get(), (unsigned char *)c->atoms.p, g, nslice, radius, vd)))
+        return rc;
     if (!vdev) CUDA_TRY(c, cudaMemcpyAsync(v_out, vd, vbytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     collect_profile(c);

@@ -144,21 +144,28 @@ struct PotArgs {
 };
 constexpr int kPotTabN = 512;   // cubic pieces per species
 constexpr int kPotMaxSp = 8;    // species the tabulated kernel takes (more: analytic kernel)
-// Atoms into slice order: atom i of slice k[i] (negative: dropped) goes to off[k] + rank[i]
-// as its nearest pixel, residue and float position (PotArgs).
+// Atoms into slice order: an atom of slice k goes to off[k] + rank as its nearest pixel,
+// residue and float position (PotArgs).
+struct alignas(16) AtomIn {
+    double x, y;
+    int k, rank, Z;
+};
 struct AtomSort {
     int natom;
-    const double *x, *y;
-    const int *Z, *k, *rank, *off;
+    const AtomIn *in;
+    const int *off;
     double ax, by, dxp, dyp;
     int nx, ny;
     int *ic, *jc, *zd;
     float *fx, *fy, *xf, *yf;
 };
 cudaError_t launch_atom_sort(const AtomSort &a, cudaStream_t s, int64_t *launches);
-// Cubic pieces of vzatom (FP64) of width h from r0 for the species whose FPARAMS rows
-// are rows[nsp][12] (device): out[nsp][kPotTabN], in t = -1/2..1/2 about each middle.
-cudaError_t launch_potential_tables(const double *rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,
+// Cubic pieces of vzatom (FP64) of width h from r0 for the species whose FPARAMS rows are
+// rows.r[nsp] (a kernel argument): out[nsp][kPotTabN], in t = -1/2..1/2 about each middle.
+struct PotRows {
+    double r[kPotMaxSp][12];
+};
+cudaError_t launch_potential_tables(const PotRows &rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,
                                     int64_t *launches);
 
 bool plan_supported(int n);

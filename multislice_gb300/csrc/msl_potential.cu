@@ -272,9 +272,10 @@ cudaError_t launch_potential(const PotArgs &a, cudaStream_t s, int64_t *launches
 namespace {
 __global__ void atom_sort_kernel(AtomSort a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.natom || a.k[i] < 0) return;
-    const int p = a.off[a.k[i]] + a.rank[i];
-    const double xw = a.x[i] - a.ax * floor(a.x[i] / a.ax), yw = a.y[i] - a.by * floor(a.y[i] / a.by);
+    if (i >= a.natom) return;
+    const AtomIn in = a.in[i];
+    const int p = a.off[in.k] + in.rank;
+    const double xw = in.x - a.ax * floor(in.x / a.ax), yw = in.y - a.by * floor(in.y / a.by);
     // nearest pixel and the FP64 residue (the same expression as |x - ix dxp| at that
     // pixel); the pixel index is then wrapped into the grid
     const double ci = floor(xw / a.dxp + 0.5), cj = floor(yw / a.dyp + 0.5);
@@ -282,7 +283,7 @@ __global__ void atom_sort_kernel(AtomSort a) {
     a.fy[p] = (float)(yw - cj * a.dyp);
     a.ic[p] = (int)ci % a.nx;
     a.jc[p] = (int)cj % a.ny;
-    a.zd[p] = a.Z[i];
+    a.zd[p] = in.Z;
     a.xf[p] = (float)xw;
     a.yf[p] = (float)yw;
 }
@@ -328,11 +329,11 @@ __device__ double vz_double(const double *f, double r) {
 }
 constexpr int TAB_THREADS = 64;
 __global__ void __launch_bounds__(TAB_THREADS)
-    potential_tables_kernel(const double *rows, double r0, double h, float4 *out) {
+    potential_tables_kernel(const __grid_constant__ PotRows rows, double r0, double h, float4 *out) {
     // four neighbouring lanes hold a piece's four points
     const int piece = (blockIdx.x * TAB_THREADS + threadIdx.x) >> 2, q = threadIdx.x & 3;
     const double r = r0 + piece * h;
-    const double y = vz_double(rows + blockIdx.y * 12, q == 0 ? r : q == 1 ? r + h / 3 : q == 2 ? r + 2 * h / 3 : r + h);
+    const double y = vz_double(rows.r[blockIdx.y], q == 0 ? r : q == 1 ? r + h / 3 : q == 2 ? r + 2 * h / 3 : r + h);
     const int l0 = threadIdx.x & 28;
     const double y0 = __shfl_sync(0xffffffffu, y, l0), y1 = __shfl_sync(0xffffffffu, y, l0 + 1),
                  y2 = __shfl_sync(0xffffffffu, y, l0 + 2), y3 = __shfl_sync(0xffffffffu, y, l0 + 3);
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(TAB_THREADS)
 }
 }  // namespace
 
-cudaError_t launch_potential_tables(const double *rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,
+cudaError_t launch_potential_tables(const PotRows &rows, int nsp, double r0, double h, float4 *out, cudaStream_t s,
                                     int64_t *launches) {
     ++*launches;
     static_assert(4 * kPotTabN % TAB_THREADS == 0, "whole blocks of pieces");

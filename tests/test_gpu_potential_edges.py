@@ -48,3 +48,21 @@ def test_atoms_just_inside_the_cutoff_of_a_tile_in_a_large_cell(ctx, fparams, nx
     ref = O.potential(x, y, z, Z, fparams, ax, by, 1.0, nx, ny, ns, radius)
     assert np.count_nonzero(ref) >= len(x)
     assert O.rel_l2(v, ref) < 1e-5
+
+
+@pytest.mark.parametrize("n,shift", [(512, 0), (513, 0), (511, 1), (512, 1), (1100, 1), (0, 0)])
+def test_more_atoms_than_the_output_holds(ctx, fparams, n, shift):
+    """Unsorted atoms pass through the output's memory: 512 of them where it is one slice
+    of 64^2 on 16 bytes, 511 where it starts 4 bytes on; then the rest."""
+    import torch
+    rng = np.random.default_rng(n)
+    ax, by, radius = 10.0, 12.0, 2.0
+    x, y, z = rng.uniform(-1, ax + 1, n), rng.uniform(-1, by + 1, n), rng.uniform(0.0, 1.0, n)
+    Z = rng.choice(np.array([8, 22, 38], np.int32), n).astype(np.int32)
+    flat = torch.full((64 * 64 + 4,), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    v = ctx.potential(S.Specimen(x, y, z, Z, ax, by, 1.0), 64, 64, 1, radius,
+                      out=flat[shift:shift + 64 * 64].view(1, 64, 64)).cpu().numpy()
+    ref = O.potential(x, y, z, Z, fparams, ax, by, 1.0, 64, 64, 1, radius)
+    assert np.abs(v - ref).max() <= 1e-5 * np.abs(ref).max()
+    assert torch.isnan(flat[:shift]).all() and torch.isnan(flat[shift + 64 * 64:]).all()

@@ -75,7 +75,8 @@ CALLS = dict(multislice=_multislice, thick=_thick, image=_image, partial=_partia
              species=_species, phonon=_phonon, jobs=_jobs, scan_384=_scan(384), scan_768=_scan(768),
              transmission=_transmission, exit=_exit)
 # bytes
-LEAST = dict(multislice=268288, thick=6792192, jobs=1363216, scan_384=3712592, transmission=398336, exit=552992)
+LEAST = dict(multislice=268288, thick=6792192, jobs=1363216, scan_384=3712592, transmission=398336, exit=552992,
+             potential=82928, species=153680)
 
 
 @pytest.mark.parametrize("call", sorted(LEAST))
