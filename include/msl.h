@@ -442,7 +442,10 @@ int msl_set_probe_batch(msl_ctx *ctx, int batch);
  * the default), for GPUs shared with other work.  A call whose buffers would
  * grow past the cap returns MSL_E_NOMEM before it frees or allocates anything
  * and leaves the context usable; the automatic probe batch of msl_stem_scan
- * shrinks to half the cap.  Caller-owned buffers are not counted.  The
+ * shrinks to half the cap.  Caller-owned buffers are not counted.  Without a cap,
+ * imaging calls (msl_ctem_image, msl_ctem_partial_coherence, msl_frozen_phonon) keep a
+ * buffer of up to 512 MB in which many images are summed at a time; under one they take
+ * one image at a time, and setting a cap gives that buffer back.  The
  * reference has no counterpart (its buffers are sized by the calculation). */
 int msl_set_memory_limit(msl_ctx *ctx, size_t bytes);
 /* Bytes the context's work buffers hold now. */

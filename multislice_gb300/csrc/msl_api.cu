@@ -529,15 +529,9 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     double psum = 0.0;
     for (double v : pw) psum += v;
     const int ndf = (int)dfs.size();
-    // one table per defocus value; then the values and the image weights, the exit intensity's last
-    const size_t tbytes = sizeof(float2) * n2 * ndf;
-    CUDA_TRY(c, c->ctf.ensure(tbytes + sizeof(double) * (2 * ndf + 1)));
+    CUDA_TRY(c, c->ctf.ensure(sizeof(float2) * n2 * ndf));  // one table per defocus value
     float2 *ctf = (float2 *)c->ctf.p;
-    double *dvals = (double *)((unsigned char *)c->ctf.p + tbytes);
-    std::vector<double> hv(dfs);
-    for (double v : pw) hv.push_back(weight * v / psum);
-    hv.push_back(weight);
-    CUDA_TRY(c, cudaMemcpyAsync(dvals, hv.data(), sizeof(double) * hv.size(), cudaMemcpyHostToDevice, c->stream));
+    for (double &v : pw) v = weight * v / psum;
     const float kob = (float)lens->k_obj;
     msl::CtfParams cp;
     cp.lam = msl_wavelength(o->kev);
@@ -549,7 +543,7 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     cp.k2obj = kob * kob;
     cp.scale = 1.0f;
     LAUNCH_TRY(c, timed(c, MSL_PROF_OTHER, [&] {
-                   return msl::launch_ctf_table(nx, ny, st.d_kx2, st.d_ky2, st.d_kx, st.d_ky, cp, dvals, ndf, ctf,
+                   return msl::launch_ctf_table(nx, ny, st.d_kx2, st.d_ky2, st.d_kx, st.d_ky, cp, dfs.data(), ndf, ctf,
                                                 c->stream, &c->launches);
                }));
     // The spectra W = Psi(k) / (nx ny) of the batch fan out to batch x ndf images, a
@@ -557,21 +551,17 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     // buffer, one row pass that adds the images in order.  One image at a time cost
     // three launches each (15 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
     const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
-    // A context with a memory cap keeps to one image's buffer.
+    // The buffer ends with the images' weights; one image's weight goes by value, so that a
+    // context with a memory cap, which keeps to one image, needs no more than it.
     size_t chunk = c->mem.limit ? 1 : std::max<size_t>(1, std::min(total, ((size_t)512 << 20) / ibytes));
-    if (c->tmpw.ensure(ibytes * chunk) != cudaSuccess) {
+    if (chunk > 1 && c->tmpw.ensure(ibytes * chunk + sizeof(double) * ndf) != cudaSuccess) {
         cudaGetLastError();
         chunk = 1;
-        CUDA_TRY(c, c->tmpw.ensure(ibytes));
     }
+    if (chunk == 1) CUDA_TRY(c, c->tmpw.ensure(ibytes));
     float2 *tmp = (float2 *)c->tmpw.p;
-    auto accumulate = [&](RowArgs &r, int nimg, int img0, const double *wt, int nw, double *acc) {
-        r.accum = acc;
-        r.accum_wt = wt;
-        r.nimg = nimg;
-        r.img0 = img0;
-        r.nw = nw;
-    };
+    double *dpw = (double *)(tmp + n2 * chunk);
+    if (chunk > 1) CUDA_TRY(c, cudaMemcpyAsync(dpw, pw.data(), sizeof(double) * ndf, cudaMemcpyHostToDevice, c->stream));
     for (size_t i0 = 0; i0 < total; i0 += chunk) {
         const int n = (int)std::min(chunk, total - i0);
         ColArgs ca = col_args(g, st, twc, 0, tmp, n, msl::COL_LOAD | msl::COL_CTF | msl::COL_INV | msl::COL_STORE,
@@ -584,7 +574,15 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
         LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, c->stream, c->nsm, &c->launches); }));
         RowArgs r = row_args(g, twr, nullptr, tmp, n, msl::ROW_LOAD | msl::ROW_INV | msl::ROW_ACCUM | msl::ROW_NOSTORE,
                              c->dflag);
-        accumulate(r, n, (int)(i0 % ndf), dvals + ndf, ndf, img_d);
+        r.accum = img_d;
+        r.nimg = n;
+        r.img0 = (int)(i0 % ndf);
+        if (chunk > 1) {
+            r.accum_wt = dpw;
+            r.nw = ndf;
+        } else {
+            r.accum_w = pw[i0 % ndf];
+        }
         LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
     }
     if (want_exit || exit_d) {  // exit waves: inverse transforms of the spectra in place
@@ -593,7 +591,9 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
         if (exit_d) {
             RowArgs r = row_args(g, twr, nullptr, w, batch,
                                  msl::ROW_LOAD | msl::ROW_INV | msl::ROW_ACCUM | msl::ROW_NOSTORE, c->dflag);
-            accumulate(r, batch, 0, dvals + 2 * ndf, 1, exit_d);
+            r.accum = exit_d;
+            r.nimg = batch;
+            r.accum_w = weight;
             LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
         }
         if (want_exit) {
@@ -1754,6 +1754,11 @@ int msl_check_wait_timeout(msl_ctx *c, uint32_t polls) {
 
 int msl_set_memory_limit(msl_ctx *c, size_t bytes) {
     if (!c) return MSL_E_ARG;
+    if (bytes && !c->mem.limit && c->tmpw.p) {  // the image buffer may be hundreds of images' until now
+        CUDA_TRY(c, cudaSetDevice(c->device));
+        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        c->tmpw.release();
+    }
     c->mem.limit = bytes;
     return MSL_OK;
 }

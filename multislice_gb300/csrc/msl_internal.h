@@ -72,10 +72,12 @@ struct RowArgs {
     float scale;           // multiplies the output when != 1
     int *err;              // set to 1 when a bounded wait gives up (may be null)
     // images onto one accumulator (ROW_LOAD [| ROW_INV] | ROW_ACCUM | ROW_NOSTORE): image i
-    // of nimg adds accum_wt[(img0 + i) % nw] * |psi|^2 to accum[nx][ny], in order
+    // of nimg adds its weight * |psi|^2 to accum[nx][ny], in order: accum_wt[(img0 + i) % nw],
+    // or accum_w for all of them (nw = 0)
     double *accum;
     int nimg, img0, nw;
     const double *accum_wt;
+    double accum_w;
     const float2 *const *trans_b;  // per-image transmission rows (replaces trans when set)
     bool shared;           // other streams' kernels run beside this one
 };
@@ -244,7 +246,7 @@ cudaError_t launch_detector_mask(int nx, int ny, const double *kxd, const double
                                  const double *kin2, const double *kout2, uint8_t *mask,
                                  cudaStream_t s, int64_t *launches);
 // ctf[ix][iy] = exp(-i chi(k)) * scale for k2 = kx2 + ky2 (float) <= k2obj, else 0;
-// chi = pi lam k2 (cs lam^2 k2 / 2 - df) in FP64, one table per defocus value df[ndf] (device)
+// chi = pi lam k2 (cs lam^2 k2 / 2 - df) in FP64, one table per defocus value df[ndf] (host)
 struct CtfParams {
     double lam, cs, dfa2, dfa2phi, dfa3, dfa3phi;
     float k2obj, scale;

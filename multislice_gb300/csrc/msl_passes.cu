@@ -121,10 +121,13 @@ __device__ __forceinline__ float2 phase_grating(float x, float s_hi, float s_lo)
     return make_float2(cn, sn);
 }
 
+__device__ __forceinline__ double image_weight(const RowArgs &a, int img) {
+    return a.nw ? a.accum_wt[(a.img0 + img) % a.nw] : a.accum_w;
+}
 // One image's share of a row's running sums; acc: this thread's first element.
 template <int T, int E>
 __device__ __forceinline__ void add_image(double (&sum)[E], const float2 (&v)[E], const RowArgs &a, int img, double *acc) {
-    const double w = a.accum_wt[(a.img0 + img) % a.nw];
+    const double w = image_weight(a, img);
     if (img == 0) {
 #pragma unroll
         for (int e = 0; e < E; ++e) sum[e] = acc[T * e];
@@ -1348,7 +1351,7 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
             for (int q = 0; q < W; ++q) {
                 const int img = r * W + q;
                 if (img < a.nimg) {
-                    const double w = a.accum_wt[(a.img0 + img) % a.nw];
+                    const double w = image_weight(a, img);
                     const float2 *x = rings + ((size_t)q * 2 + ((done * ((a.nimg - q + W - 1) / W) + r) & 1)) * UNIT;
 #pragma unroll
                     for (int i = 0; i < PX; ++i) {
@@ -1620,8 +1623,12 @@ __global__ void detector_mask_kernel(int nx, int ny, const double *kxd, const do
     mask[(size_t)ix * ny + iy] = (uint8_t)bits;
 }
 
+constexpr int kDfBatch = 256;  // defocus values a launch
+struct DfList {
+    double v[kDfBatch];
+};
 __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
-                                 const float *ky, CtfParams p, const double *df, float2 *ctf) {
+                                 const float *ky, CtfParams p, const __grid_constant__ DfList df, float2 *ctf) {
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int ix = blockIdx.y;
     if (iy >= ny || ix >= nx) return;
@@ -1629,7 +1636,7 @@ __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *
     float2 out = make_float2(0.f, 0.f);
     if (k2 <= p.k2obj) {
         const double q = (double)k2;
-        double w = 0.5 * p.cs * p.lam * p.lam * q - df[blockIdx.z];
+        double w = 0.5 * p.cs * p.lam * p.lam * q - df.v[blockIdx.z];
         if (p.dfa2 != 0.0 || p.dfa3 != 0.0) {
             const double phi = atan2((double)ky[iy], (double)kx[ix]);
             w += p.dfa2 * sin(2.0 * (phi - p.dfa2phi)) +
@@ -2270,9 +2277,14 @@ cudaError_t launch_detector_mask(int nx, int ny, const double *kxd, const double
 cudaError_t launch_ctf_table(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
                              const float *ky, const CtfParams &p, const double *df, int ndf, float2 *ctf,
                              cudaStream_t s, int64_t *launches) {
-    ++*launches;
-    dim3 grid((ny + 255) / 256, nx, ndf);
-    ctf_table_kernel<<<grid, 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, df, ctf);
+    for (int j = 0; j < ndf; j += kDfBatch) {
+        DfList l;
+        const int n = ndf - j < kDfBatch ? ndf - j : kDfBatch;
+        memcpy(l.v, df + j, sizeof(double) * n);
+        ++*launches;
+        ctf_table_kernel<<<dim3((ny + 255) / 256, nx, n), 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, l,
+                                                                      ctf + (size_t)j * nx * ny);
+    }
     return cudaGetLastError();
 }
 

@@ -76,7 +76,7 @@ CALLS = dict(multislice=_multislice, thick=_thick, image=_image, partial=_partia
              transmission=_transmission, exit=_exit)
 # bytes
 LEAST = dict(multislice=268288, thick=6792192, jobs=1363216, scan_384=3712592, transmission=398336, exit=552992,
-             potential=82928, species=153680)
+             potential=82928, species=153680, phonon=289340, image=591872, partial=756296)
 
 
 @pytest.mark.parametrize("call", sorted(LEAST))
@@ -88,3 +88,17 @@ def test_runs_in_the_cap_it_always_ran_in(call):
         c.set_memory_limit(LEAST[call])
         assert np.array_equal(CALLS[call](c), free)
         assert c.memory_in_use() <= LEAST[call]
+
+
+def test_a_cap_gives_the_image_buffer_back():
+    """Images are summed up to 512 MB at a time without a cap; the buffer that takes
+    does not stand in the way of a cap set later."""
+    from multislice_gb300 import Context
+    n, cap = 512, 64 << 20
+    with Context(0) as c:
+        c.ctem_image(_t(1, n), 1.5, [0], 30.0, 30.0, 200.0, 1.2e7, -600.0, 1.5, batch=16, df_spread=8.0, df_step=20.0)
+        assert c.memory_in_use() > cap
+        c.set_memory_limit(cap)
+        assert c.memory_in_use() <= cap
+        v = c.potential(S.srtio3(8, 8, 4), n, n, 2, 3.0)
+        assert np.isfinite(v).all() and c.memory_in_use() <= cap
