@@ -796,7 +796,9 @@ __global__ void __launch_bounds__(128, ColMixedCfg<N>::MINB)
         }
         if (a.flags & COL_PROP) col_propagate<M>(u, a, b, iy, uj);
         if (a.flags & COL_CTF) col_ctf<M>(u, a, b, iy, uj);
-        if (a.flags & COL_DETECT) col_detect<M, Cfg::NWARP>(u, a, b, iy, uj, ty, tpi, red);
+        if constexpr (N == 384) {  // at 768 these passes go elsewhere (launch_col_pass)
+            if (a.flags & COL_DETECT) col_detect<M, Cfg::NWARP>(u, a, b, iy, uj, ty, tpi, red);
+        }
         if (a.flags & COL_INV) mixed_from24<M, -1, QV>(u, v, vj, uj, at, at, tb, ctasync);
         if (store) {
             __syncthreads();  // every thread is done reading the slot
@@ -1798,6 +1800,7 @@ static bool col_maps(const ColArgs &a, int n, int c, int boxr, CUtensorMap *load
 
 template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStream_t s, int nsm) {
     using Cfg = ColMixedCfg<N>;
+    static_assert(N != 384 || Cfg::C == ColPlan<N>::col_c, "detector partials per ColPlan's tile");
     static KernelSetup ks;
     int per_sm = 0;
     cudaError_t e = ks.get(col_mixed_kernel<N>, Cfg::THREADS, Cfg::SMEM, true, &per_sm);
@@ -2016,8 +2019,6 @@ int plan_col_c_launch(int n, const ColArgs &a) {
         ColArgs f = a;
         f.flags = (f.flags | COL_LOAD | COL_FWD) & ~COL_PROBE;
         if (fam == FAM_FAST && col_half_side(n, f)) return 4;
-        if (fam == FAM_FAST && n == 384) return ColMixedCfg<384>::C;
-        if (fam == FAM_FAST && n == 768) return ColMixedCfg<768>::C;
         switch (n) {
 #define X(N) case N: return ColPlan<N>::col_c;
             MSL_FOR_EACH_SIDE(X)
@@ -2211,9 +2212,12 @@ cudaError_t launch_col_pass(int nx, const ColArgs &a, cudaStream_t s, int nsm, i
             case 1024: return col_half_launch<ColPairL1024>(a, s, nsm);
             default: break;
         }
-        if (fam == FAM_FAST && (a.flags & COL_LOAD)) {  // 384 and 768: two-stage columns for every loaded pass
+        // 384 and 768: two-stage columns for every loaded pass, but not for a scan's detector
+        // sums at 768, whose partials (one per tile of 4 columns instead of 8) would take
+        // twice the scratch: such a pass is 0.31 ms instead of 0.28 at 128 waves
+        if (fam == FAM_FAST && (a.flags & COL_LOAD)) {
             if (nx == 384) return col_mixed_launch<384>(a, s, nsm);
-            if (nx == 768) return col_mixed_launch<768>(a, s, nsm);
+            if (nx == 768 && !(a.flags & COL_DETECT)) return col_mixed_launch<768>(a, s, nsm);
         }
         switch (nx) {
 #define X(N) case N: return col_tma_launch<N>(a, s, nsm);
