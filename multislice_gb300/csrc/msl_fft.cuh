@@ -776,6 +776,7 @@ template <int N_> struct Mixed {
     static constexpr int N = N_, RB = N_ / 24, T = RB, E = 24;
     static constexpr int QV_ROW = RB == 16 ? 2 : 1;  // radix-RB butterflies a thread holds
     static constexpr int PA = RB + 1, PB = 25, SLOTS = 24 * PA > RB * PB ? 24 * PA : RB * PB;
+    static constexpr int GTW_OFF = plan_tw_size<Plan<N_>>();  // exp(2 pi i r k / N), [24][RB], after Plan's tables
     static constexpr bool PK = true;
     static_assert(N == 384 || N == 768, "sides of the two-stage mixed plans");
 };

@@ -55,11 +55,13 @@ constexpr size_t kOffKy2 = kOffKx2 + sizeof(float) * kMaxSide;
 constexpr size_t kOffProp = kOffKy2 + sizeof(float) * kMaxSide;
 constexpr size_t kScratchBytes = kOffProp + sizeof(float2) * (size_t)kMaxLayers * 2 * kMaxSide;
 static_assert(kScratchBytes == MSL_NOALLOC_SCRATCH_BYTES, "scratch size must match msl.h");
-// every side's twiddle buffer (with the two-stage 1024 row table appended) fits its slot
+// every side's twiddle buffer (with the two-stage tables of 384, 768 and 1024 appended) fits its slot
 #define X(N) static_assert(msl::plan_tw_size<msl::Plan<N>>() <= kMaxTw, "twiddle slot too small for side " #N);
 MSL_FOR_EACH_SIDE(X)
 #undef X
-static_assert(msl::WarpPlan1024x2::GTW_OFF + 32 * 32 <= kMaxTw, "the 1024 buffer holds the two-stage row table");
+static_assert(msl::WarpPlan1024x2::GTW_OFF + 32 * 32 <= kMaxTw && msl::Mixed<384>::GTW_OFF + 384 <= kMaxTw &&
+                  msl::Mixed<768>::GTW_OFF + 768 <= kMaxTw,
+              "the buffers hold the two-stage tables");
 static_assert(kOffTwCol % 256 == 0 && kOffKx2 % 256 == 0 && kOffProp % 256 == 0, "alignment");
 
 std::mutex g_mu;

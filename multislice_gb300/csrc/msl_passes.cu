@@ -692,15 +692,13 @@ __global__ void __launch_bounds__(ColHalfCfg<L>::THREADS, 1)
     }
 }
 
-// exp(2 pi i r k / N) at [r][k], r < 24, k < RB, then r < RB, k < 24
-template <int N> __device__ __forceinline__ void mixed_tables(float2 *t) {
+// exp(2 pi i r k / N) at [r][k], r < 24, k < RB, then r < RB, k < 24, from the host's table
+// (formed here from a rounded quotient r k / N they were up to 2e-7 rad off, and 768^2
+// exit waves 8 % further from FP64 than with the three-stage plans)
+template <int N> __device__ __forceinline__ void mixed_tables(float2 *t, const float2 *__restrict__ tw) {
     constexpr int RB = Mixed<N>::RB;
-    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) {
-        const int j = i % N, m = i < N ? (j / RB) * (j % RB) : (j / 24) * (j % 24);
-        float sn, cn;
-        sincospif((float)(2 * m) / (float)N, &sn, &cn);
-        t[i] = make_float2(cn, sn);
-    }
+    tw += Mixed<N>::GTW_OFF;
+    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) t[i] = tw[i < N ? i : (i - N) % 24 * RB + (i - N) / 24];
 }
 
 // ---------------------------------------- two-stage column pass, 384 and 768
@@ -738,7 +736,7 @@ __global__ void __launch_bounds__(128, ColMixedCfg<N>::MINB)
     int vj[QV];
 #pragma unroll
     for (int q = 0; q < QV; ++q) vj[q] = uj + RB * q;
-    mixed_tables<N>(t24);
+    mixed_tables<N>(t24, a.tw);
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -992,7 +990,7 @@ __global__ void __launch_bounds__(RowMixedCfg<N>::THREADS, IMG ? 1 : RowMixedCfg
     unsigned char *ring = base + warp * 2 * Cfg::SLOT;
     float2 *t24 = reinterpret_cast<float2 *>(base + Cfg::OFF_T), *tb = t24 + N;
     uint64_t *bar = reinterpret_cast<uint64_t *>(base + Cfg::OFF_BAR) + warp * 2;
-    mixed_tables<N>(t24);
+    mixed_tables<N>(t24, a.tw);
     if (lane == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -2084,19 +2082,28 @@ int plan_twiddles_into(int n, float2 *out, int cap) {
 }
 
 int row_two_twiddles_size(int n) {
-    return n == WarpPlan1024x2::N && WarpPlan1024x2::GTW ? WarpPlan1024x2::GTW_OFF + 32 * 32 : 0;
+    switch (n) {
+        case 384: return Mixed<384>::GTW_OFF + 384;
+        case 768: return Mixed<768>::GTW_OFF + 768;
+        case WarpPlan1024x2::N: return WarpPlan1024x2::GTW_OFF + 32 * 32;
+        default: return 0;
+    }
 }
 
 void append_row_two_twiddles(int n, float2 *tables) {
-    if (!row_two_twiddles_size(n)) return;
-    // the two-stage 1024 row plan's stage-1 table [r][k] = exp(2 pi i r k / 1024),
-    // r, k < 32, after Plan<1024>'s own tables (read through L1 by the row kernel)
-    using P = WarpPlan1024x2;
-    for (int r = 0; r < 32; ++r)
-        for (int k = 0; k < 32; ++k) {
-            const double ph = 2.0 * 3.14159265358979323846 * (double)((r * k) % 1024) / 1024.0;
-            tables[(size_t)P::GTW_OFF + r * 32 + k] = make_float2((float)cos(ph), (float)sin(ph));
-        }
+    const int size = row_two_twiddles_size(n);
+    if (!size) return;
+    // the two-stage plan's table [r][k] = exp(2 pi i r k / n), after Plan<n>'s own: 1024
+    // rows r, k < 32 (read through L1 by the row kernel); 384 and 768 r < 24, k < n / 24
+    const int nk = n == 1024 ? 32 : n / 24, count = n == 1024 ? 32 * 32 : n;
+    // the float constants of the radix 8, 16, 24 and 32 butterflies lie below the exact
+    // ones and take 2.5e-8 (384) or 3.0e-8 (768) of a line's amplitude, the same in every
+    // slice: the factors of 384 and 768 put it back (1024's are as they always were)
+    const double unit = n == 384 ? 1.0 + 2.0e-8 : n == 768 ? 1.0 + 2.8e-8 : 1.0;
+    for (int i = 0; i < count; ++i) {
+        const double ph = 2.0 * 3.14159265358979323846 * (double)(((i / nk) * (i % nk)) % n) / n;
+        tables[size - count + i] = make_float2((float)(unit * cos(ph)), (float)(unit * sin(ph)));
+    }
 }
 
 // The slice loop's row pass (load, inverse, * t, forward, store) on the tensor cores.
