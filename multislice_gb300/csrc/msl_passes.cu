@@ -85,12 +85,10 @@ static cudaError_t launch_pass(void (*kern)(KA...), int grid, dim3 block, size_t
 //   1024^2:  256 MB 252 / 253 us, 384 MB 368 / 365, 512 MB 503 / 478, 4 GB 5.41 / 4.33 ms
 //    768^2:  288 MB 283 / 285 us, 432 MB 416 / 415, 864 MB 905 / 803
 //    512^2 scan:   2 GB 1.60 / 1.60 ms, 8 GB 6.69 / 6.31;   256^2 and 2048^2, 4 GB: + 1 %
-// At 384 the same is seen from 28 MB on (72 MB 86 / 76 us, 96 MB 106 / 98; 16 MB 25 / 26;
-// 160 MB and more 2 % the other way).  Row passes, whose lines are their own, overlap at
-// any size.
+// (384 and 768 besides: mixed_overlaps).  Row passes, whose lines are their own, overlap
+// at any size.
 static bool col_overlaps(const ColArgs &a, int nx) {
-    const size_t limit = (size_t)(nx == 384 ? 20 : 320) << 20;
-    return !a.shared && sizeof(float2) * a.batch * a.ny * nx <= limit;
+    return !a.shared && sizeof(float2) * a.batch * a.ny * nx <= (size_t)320 << 20;
 }
 
 // CTAs a pass of `units` independent pieces of work is spread over, each CTA able to
@@ -1796,6 +1794,21 @@ static bool col_maps(const ColArgs &a, int n, int c, int boxr, CUtensorMap *load
     return !a.fan || encode(load, a.in, (a.img0 + a.batch - 1) / a.fan + 1);
 }
 
+// Whether the two-stage columns of a side overlap at all, three CTAs an SM with a few
+// tiles each.  A plain launch gives every SM one CTA, then a second and a third, so a last
+// round that only some CTAs have is spread over all SMs; as dependents the CTAs go where
+// there is room first, and past one an SM the last round's pile up there.  From some
+// rounds on (13 of 384, 5 of 768) its share no longer matters; below two the overlapped
+// start gains more.  Overlapped against plain, a slice step, by rounds:
+//   384:  1.89 - 5 %, 2.53 + 8 %, 4.63 + 16 %, 5.05 - 4 %, 5.16 + 4 %, 5.47 + 20 %, 6.32 - 4 %, 6.42 + 10 %,
+//         8.21 - 3 %, 8.42 + 16 %, 9.05 - 2 %, 10.74 + 4 %, 12.21 - 2 %, 12.74 + 2 %, 15.2 - 2 %, 27 - 1 %
+//   768:  1.68 - 1 %, 2.11 + 8 %, 3.37 + 8 %, 4.21 - 5 %, 4.63 + 8 %, 5.05 - 4 %, 5.47 - 4 %, 9.26 - 2 %
+static bool mixed_overlaps(int tiles, int ctas, int nsm, int n) {
+    const int rounds = tiles / ctas;
+    if (rounds < 2 || rounds >= (n == 384 ? 13 : 5)) return true;
+    return rounds >= (n == 384 ? 6 : 4) && tiles % ctas <= nsm;
+}
+
 template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStream_t s, int nsm) {
     using Cfg = ColMixedCfg<N>;
     static_assert(N != 384 || Cfg::C == ColPlan<N>::col_c, "detector partials per ColPlan's tile");
@@ -1807,7 +1820,8 @@ template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStrea
     if (!col_maps(a, N, Cfg::C, Cfg::BOXR, &map, &mapo)) return cudaErrorInvalidValue;
     const int ntiles = a.batch * (a.ny / Cfg::C);
     const int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
-    return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, col_overlaps(a, N), map, mapo, a);
+    const bool alone = col_overlaps(a, N) && mixed_overlaps(ntiles, nsm * per_sm, nsm, N);
+    return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, alone, map, mapo, a);
 }
 
 template <class PL, int MINB> static cudaError_t col_tma_launch_v(const ColArgs &a, cudaStream_t s, int nsm) {
