@@ -384,8 +384,6 @@ template <class P> struct RowXorLin {
     uint32_t base;  // shared address of the line, aligned to N * 8 bytes
     static __host__ __device__ constexpr int f(int i) { return i ^ ((i >> P::row_sh) & 15); }
 };
-template <class A> struct is_xor_lin { static constexpr bool value = false; };
-template <class P> struct is_xor_lin<RowXorLin<P>> { static constexpr bool value = true; };
 
 __device__ __forceinline__ void sts_f2(uint32_t addr, float2 v) {
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
@@ -487,13 +485,10 @@ __device__ __forceinline__ void fft_stage_cw(float2 (&v)[P::E], int t, const flo
     }
 }
 
-// WARP = true: the line belongs to one warp (T == 32) and the exchange needs
-// only warp-level synchronisation.
-template <class P, int S, bool WARP = false, class Addr>
+template <class P, int S, class Addr>
 __device__ __forceinline__ void fft_exchange(float2 (&v)[P::E], int t, const Addr &ad) {
     constexpr int R = P::radix(S), NS = plan_span<P>(S), E = P::E, Q = E / R, T = P::T;
-    static_assert(!WARP || T == 32 || T == 16, "warp-owned lines: 32 threads per line, or two half-warp lines");
-    if constexpr (WARP) __syncwarp(); else __syncthreads();  // previous readers are done
+    __syncthreads();  // previous readers are done
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int j = t + T * q;
@@ -501,7 +496,7 @@ __device__ __forceinline__ void fft_exchange(float2 (&v)[P::E], int t, const Add
 #pragma unroll
         for (int r = 0; r < R; ++r) ad.base[ad(d + r * NS)] = v[q + r * Q];
     }
-    if constexpr (WARP) __syncwarp(); else __syncthreads();
+    __syncthreads();
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = ad.base[ad(t + T * e)];
 }
@@ -579,16 +574,14 @@ __device__ __forceinline__ void fft_exchange_cl(float2 (&v)[P::E], int t, const 
     }
 }
 
-template <class P, int DIR, int S = 0, bool WARP = false, class Addr>
+template <class P, int DIR, int S = 0, class Addr>
 __device__ __forceinline__ void fft_line(float2 (&v)[P::E], int t, const Addr &ad,
                                          const float2 *__restrict__ tw) {
-    if constexpr (is_xor_lin<Addr>::value) fft_stage_cw<P, S, DIR>(v, t, tw);
-    else fft_stage<P, S, DIR>(v, t, tw);
+    fft_stage<P, S, DIR>(v, t, tw);
     if constexpr (S + 1 < P::NSTAGE) {
-        if constexpr (is_xor_lin<Addr>::value) fft_exchange_xl<P, S>(v, t, ad);
-        else if constexpr (is_col_lin<Addr>::value) fft_exchange_cl<P, S>(v, t, ad);
-        else fft_exchange<P, S, WARP>(v, t, ad);
-        fft_line<P, DIR, S + 1, WARP>(v, t, ad, tw);
+        if constexpr (is_col_lin<Addr>::value) fft_exchange_cl<P, S>(v, t, ad);
+        else fft_exchange<P, S>(v, t, ad);
+        fft_line<P, DIR, S + 1>(v, t, ad, tw);
     }
 }
 

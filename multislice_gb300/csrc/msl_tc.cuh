@@ -53,9 +53,6 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
-// What N columns add to an instruction descriptor.
-__host__ __device__ constexpr uint32_t idesc_n(int N) { return (uint32_t)(N >> 3) << 17; }
-
 // TMEM allocation by one full warp; the base address is written to *dst (shared).
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
