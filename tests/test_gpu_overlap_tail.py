@@ -1,6 +1,7 @@
-"""Two-stage columns of 384 and 768 launched as dependents or plainly by how full their
-last round of tiles is: a wave of a batch on either side of each line (of a GPU of 152
-SMs) equals its own run."""
+"""Columns launched as dependents or plainly by the size of the waves and, two-stage ones
+of 384 and 768, by how full their last round of tiles is; 256^2 tiles dealt differently
+past 65536: a wave of a batch on either side of each line (of a GPU of 152 SMs) equals
+its own run, all inputs made before the calls."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,batch", [(384, 18), (384, 19), (384, 56), (384, 57), (384, 60), (384, 61), (384, 123),
-                                     (384, 124), (768, 4), (768, 5), (768, 9), (768, 10), (768, 11), (768, 12)])
+                                     (384, 124), (768, 4), (768, 5), (768, 9), (768, 10), (768, 11), (768, 12), (768, 71), (768, 72), (256, 2047),
+                                     (256, 2048), (1024, 40), (1024, 41)])
 def test_batches_on_both_sides_of_the_rounds(n, batch):
     from multislice_gb300 import Context
     g = torch.Generator(device="cuda").manual_seed(n + batch)
