@@ -95,8 +95,8 @@ int msl_ctx_destroy(msl_ctx *ctx);
 const char *msl_last_error(const msl_ctx *ctx);
 /* Library version string. */
 const char *msl_version(void);
-/* Number of kernels this context has launched since creation (the one that turns a
- * call's uploaded frequencies into its propagator tables not counted). */
+/* Number of kernels this context has launched since creation (those that turn a call's
+ * slice thicknesses into its propagator tables, part of its set-up, not counted). */
 int64_t msl_kernel_launches(const msl_ctx *ctx);
 
 /* ------------------------------------------------------------ parameters */

@@ -549,7 +549,7 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     // The spectra W = Psi(k) / (nx ny) of the batch fan out to batch x ndf images, a
     // chunk at a time: one column pass (times the table, inverse) into the chunk's
     // buffer, one row pass that adds the images in order.  One image at a time cost
-    // three launches each (15 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
+    // three launches each (13 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
     const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
     // The buffer ends with the images' weights; one image's weight goes by value, so that a
     // context with a memory cap, which keeps to one image, needs no more than it.
@@ -1644,7 +1644,7 @@ int msl_run_jobs(msl_ctx *c, const msl_job *jobs, int njobs, double bandlimit) {
         groups.push_back(std::move(g));
     }
     // The group with the most work (the longest chain of passes) last: its stream's CTAs
-    // go first and the others fill in (the batch of 20 jobs: 4.33 -> 4.1 ms).
+    // go first and the others fill in (20 jobs of sides 256 to 1024: 3.99 -> 3.74 ms).
     auto cost = [&](const JobGroup &g) {
         double s = 0;
         for (int j : g.ids) s += (double)g.nx * g.ny * jobs[j].nslice;

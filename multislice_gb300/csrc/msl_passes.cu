@@ -55,7 +55,7 @@ template <int N> struct ColCfg {
 // launched one after the other (the uneven batch: 4.5 ms plain, 6.4 ms overlapped).
 // So are the image sums: CTAs let in early gather on the SMs that have room at that
 // moment, and a long kernel of fewer CTAs than SMs then waits for the fullest one
-// (165 images of 256^2: 0.14 ms plain, 0.52 ms overlapped).
+// (143 images of 256^2: 0.14 ms plain, 0.52 ms overlapped).
 // Si 256^2, one wave, 161 passes: 1.20 -> 0.66 ms a call, with the work spread (below).
 __device__ __forceinline__ void pass_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1273,7 +1273,7 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, RowTwoCfg<P>::MINB) row
 // a time; the intensities then go through shared memory and every thread adds the four
 // images, in order, to the FP64 sums it keeps in registers.  The image order is fixed,
 // so the sums do not depend on how images are grouped into launches.  One warp walking
-// all images by itself left an SM with one warp's latencies: 165 images of 256^2 in
+// all images by itself left an SM with one warp's latencies: 143 images of 256^2 in
 // 502 us, now 139 us (two thirds of the FP64 pipe).
 template <class P>
 __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(RowArgs a) {
