@@ -494,25 +494,6 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     int rc;
     const int nx = g->nx, ny = g->ny;
     const size_t n2 = (size_t)nx * ny;
-    SliceTables st;
-    if ((rc = build_slice_tables(c, g, o, ntrans, dz, st))) return rc;
-    float2 *twr = twiddles(c, ny), *twc = twiddles(c, nx);
-    if (!twr || !twc) return fail(c, MSL_E_NOMEM, "twiddle table allocation failed");
-    for (int s = 0; s < nslice; ++s) {
-        const int l = seq[s];
-        int rf = msl::ROW_TRANS | msl::ROW_FWD;
-        if (s > 0) rf |= msl::ROW_LOAD | msl::ROW_INV;
-        else if (!plane) rf |= msl::ROW_LOAD;
-        // ttab: every image its own transmission, [slice step][image] row pointers
-        RowArgs r = row_args(g, twr, ttab ? nullptr : td + (size_t)l * n2, w, batch, rf, c->dflag);
-        if (ttab) r.trans_b = ttab + (size_t)s * batch;
-        LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
-        // the last slice keeps the spectrum: W = Psi(k) / (nx ny) after the propagator
-        int cf = msl::COL_LOAD | msl::COL_FWD | msl::COL_PROP | msl::COL_STORE;
-        if (s + 1 < nslice) cf |= msl::COL_INV;
-        ColArgs ca = col_args(g, st, twc, l, w, batch, cf, c->dflag);
-        LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, c->stream, c->nsm, &c->launches); }));
-    }
     // defocus values and weights (mulslice.cpp:552, :610-642)
     std::vector<double> dfs, pw;
     if (lens->df_spread > 0) {
@@ -532,6 +513,39 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     CUDA_TRY(c, c->ctf.ensure(sizeof(float2) * n2 * ndf));  // one table per defocus value
     float2 *ctf = (float2 *)c->ctf.p;
     for (double &v : pw) v = weight * v / psum;
+    const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
+    // Images are summed a chunk at a time.  Their buffer ends with the images' weights; one
+    // weight goes by value, so that a context with a memory cap, which keeps to one image,
+    // needs no more than it.
+    size_t chunk = c->mem.limit ? 1 : std::max<size_t>(1, std::min(total, ((size_t)512 << 20) / ibytes));
+    if (chunk > 1 && c->tmpw.ensure(ibytes * chunk + (ndf > 1 ? sizeof(double) * ndf : 0)) != cudaSuccess) {
+        cudaGetLastError();
+        chunk = 1;
+    }
+    if (chunk == 1) CUDA_TRY(c, c->tmpw.ensure(ibytes));
+    float2 *tmp = (float2 *)c->tmpw.p;
+    double *dpw = (double *)(tmp + n2 * chunk);
+    const bool many = chunk > 1 && ndf > 1;  // weights on the device, copied before anything runs
+    if (many) CUDA_TRY(c, cudaMemcpyAsync(dpw, pw.data(), sizeof(double) * ndf, cudaMemcpyHostToDevice, c->stream));
+    SliceTables st;
+    if ((rc = build_slice_tables(c, g, o, ntrans, dz, st))) return rc;
+    float2 *twr = twiddles(c, ny), *twc = twiddles(c, nx);
+    if (!twr || !twc) return fail(c, MSL_E_NOMEM, "twiddle table allocation failed");
+    for (int s = 0; s < nslice; ++s) {
+        const int l = seq[s];
+        int rf = msl::ROW_TRANS | msl::ROW_FWD;
+        if (s > 0) rf |= msl::ROW_LOAD | msl::ROW_INV;
+        else if (!plane) rf |= msl::ROW_LOAD;
+        // ttab: every image its own transmission, [slice step][image] row pointers
+        RowArgs r = row_args(g, twr, ttab ? nullptr : td + (size_t)l * n2, w, batch, rf, c->dflag);
+        if (ttab) r.trans_b = ttab + (size_t)s * batch;
+        LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
+        // the last slice keeps the spectrum: W = Psi(k) / (nx ny) after the propagator
+        int cf = msl::COL_LOAD | msl::COL_FWD | msl::COL_PROP | msl::COL_STORE;
+        if (s + 1 < nslice) cf |= msl::COL_INV;
+        ColArgs ca = col_args(g, st, twc, l, w, batch, cf, c->dflag);
+        LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, c->stream, c->nsm, &c->launches); }));
+    }
     const float kob = (float)lens->k_obj;
     msl::CtfParams cp;
     cp.lam = msl_wavelength(o->kev);
@@ -550,18 +564,6 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     // chunk at a time: one column pass (times the table, inverse) into the chunk's
     // buffer, one row pass that adds the images in order.  One image at a time cost
     // three launches each (13 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
-    const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
-    // The buffer ends with the images' weights; one image's weight goes by value, so that a
-    // context with a memory cap, which keeps to one image, needs no more than it.
-    size_t chunk = c->mem.limit ? 1 : std::max<size_t>(1, std::min(total, ((size_t)512 << 20) / ibytes));
-    if (chunk > 1 && c->tmpw.ensure(ibytes * chunk + sizeof(double) * ndf) != cudaSuccess) {
-        cudaGetLastError();
-        chunk = 1;
-    }
-    if (chunk == 1) CUDA_TRY(c, c->tmpw.ensure(ibytes));
-    float2 *tmp = (float2 *)c->tmpw.p;
-    double *dpw = (double *)(tmp + n2 * chunk);
-    if (chunk > 1) CUDA_TRY(c, cudaMemcpyAsync(dpw, pw.data(), sizeof(double) * ndf, cudaMemcpyHostToDevice, c->stream));
     for (size_t i0 = 0; i0 < total; i0 += chunk) {
         const int n = (int)std::min(chunk, total - i0);
         ColArgs ca = col_args(g, st, twc, 0, tmp, n, msl::COL_LOAD | msl::COL_CTF | msl::COL_INV | msl::COL_STORE,
@@ -577,7 +579,7 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
         r.accum = img_d;
         r.nimg = n;
         r.img0 = (int)(i0 % ndf);
-        if (chunk > 1) {
+        if (many) {
             r.accum_wt = dpw;
             r.nw = ndf;
         } else {

@@ -1323,6 +1323,9 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
             if (lane == 0 && r + 1 < rounds) issue(r + 1);
             const bool mine = r * W + warp < a.nimg;
             bool got = true;
+            double wt[W];  // the round's weights, fetched while its lines are transformed
+#pragma unroll
+            for (int q = 0; q < W; ++q) wt[q] = r * W + q < a.nimg ? image_weight(a, r * W + q) : 0.0;
             if (mine) {
                 float2 *buf = ring + (used & 1u) * UNIT + h * N;
                 got = mbar_wait_bounded(&bar[used & 1u], (used >> 1) & 1u, kWaitLimit);
@@ -1349,12 +1352,11 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
             for (int q = 0; q < W; ++q) {
                 const int img = r * W + q;
                 if (img < a.nimg) {
-                    const double w = image_weight(a, img);
                     const float2 *x = rings + ((size_t)q * 2 + ((done * ((a.nimg - q + W - 1) / W) + r) & 1)) * UNIT;
 #pragma unroll
                     for (int i = 0; i < PX; ++i) {
                         const float2 v = x[tid + Cfg::THREADS * i];
-                        sum[i] += w * ((double)v.x * v.x + (double)v.y * v.y);
+                        sum[i] += wt[q] * ((double)v.x * v.x + (double)v.y * v.y);
                     }
                 }
             }
@@ -1621,12 +1623,12 @@ __global__ void detector_mask_kernel(int nx, int ny, const double *kxd, const do
     mask[(size_t)ix * ny + iy] = (uint8_t)bits;
 }
 
-constexpr int kDfBatch = 256;  // defocus values a launch
-struct DfList {
-    double v[kDfBatch];
+template <int CAP> struct DfList {
+    double v[CAP];
 };
+template <int CAP>
 __global__ void ctf_table_kernel(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
-                                 const float *ky, CtfParams p, const __grid_constant__ DfList df, float2 *ctf) {
+                                 const float *ky, CtfParams p, const __grid_constant__ DfList<CAP> df, float2 *ctf) {
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int ix = blockIdx.y;
     if (iy >= ny || ix >= nx) return;
@@ -2262,7 +2264,7 @@ static void prop_tables_v(const PropTable *tabs, int n, int nx, int ny, float2 *
     prop_table_kernel<CAP><<<dim3((nx + ny + 127) / 128, n), 128, 0, s>>>(a, nx, ny, 1.0f / ((float)nx * (float)ny), out);
 }
 cudaError_t launch_prop_tables(const PropTable *tabs, int ntab, int nx, int ny, float2 *out, cudaStream_t s) {
-    constexpr int kFew = 32, kMany = 512;  // 1.3 and 20 KB of arguments (of 32)
+    constexpr int kFew = 16, kMany = 512;  // 0.6 and 20 KB of arguments (of 32)
     for (int t = 0; t < ntab; t += kMany) {
         const int n = ntab - t < kMany ? ntab - t : kMany;
         float2 *o = out + (size_t)t * (nx + ny);
@@ -2299,16 +2301,23 @@ cudaError_t launch_detector_mask(int nx, int ny, const double *kxd, const double
     return cudaGetLastError();
 }
 
+template <int CAP>
+static void ctf_tables_v(int nx, int ny, const float *kx2, const float *ky2, const float *kx, const float *ky,
+                         const CtfParams &p, const double *df, int n, float2 *ctf, cudaStream_t s) {
+    DfList<CAP> l;
+    memcpy(l.v, df, sizeof(double) * n);
+    ctf_table_kernel<CAP><<<dim3((ny + 255) / 256, nx, n), 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, l, ctf);
+}
 cudaError_t launch_ctf_table(int nx, int ny, const float *kx2, const float *ky2, const float *kx,
                              const float *ky, const CtfParams &p, const double *df, int ndf, float2 *ctf,
                              cudaStream_t s, int64_t *launches) {
-    for (int j = 0; j < ndf; j += kDfBatch) {
-        DfList l;
-        const int n = ndf - j < kDfBatch ? ndf - j : kDfBatch;
-        memcpy(l.v, df + j, sizeof(double) * n);
+    constexpr int kFew = 16, kMany = 256;
+    for (int j = 0; j < ndf; j += kMany) {
+        const int n = ndf - j < kMany ? ndf - j : kMany;
+        float2 *t = ctf + (size_t)j * nx * ny;
         ++*launches;
-        ctf_table_kernel<<<dim3((ny + 255) / 256, nx, n), 256, 0, s>>>(nx, ny, kx2, ky2, kx, ky, p, l,
-                                                                      ctf + (size_t)j * nx * ny);
+        if (n <= kFew) ctf_tables_v<kFew>(nx, ny, kx2, ky2, kx, ky, p, df + j, n, t, s);
+        else ctf_tables_v<kMany>(nx, ny, kx2, ky2, kx, ky, p, df + j, n, t, s);
     }
     return cudaGetLastError();
 }
