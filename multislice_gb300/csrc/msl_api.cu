@@ -494,6 +494,10 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     int rc;
     const int nx = g->nx, ny = g->ny;
     const size_t n2 = (size_t)nx * ny;
+    SliceTables st;
+    if ((rc = build_slice_tables(c, g, o, ntrans, dz, st))) return rc;
+    float2 *twr = twiddles(c, ny), *twc = twiddles(c, nx);
+    if (!twr || !twc) return fail(c, MSL_E_NOMEM, "twiddle table allocation failed");
     // defocus values and weights (mulslice.cpp:552, :610-642)
     std::vector<double> dfs, pw;
     if (lens->df_spread > 0) {
@@ -514,23 +518,20 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     float2 *ctf = (float2 *)c->ctf.p;
     for (double &v : pw) v = weight * v / psum;
     const size_t total = (size_t)batch * ndf, ibytes = sizeof(float2) * n2;
-    // Images are summed a chunk at a time.  Their buffer ends with the images' weights; one
-    // weight goes by value, so that a context with a memory cap, which keeps to one image,
-    // needs no more than it.
+    pw.push_back(weight);  // of the exit intensity
+    // Images are summed a chunk at a time, a single one at a time in a context with a
+    // memory cap.  Their weights lie where the propagator tables were, without scratch of
+    // their own; where they are too many for that (many defocus values, few layers), behind
+    // the chunk's images, or under a cap as many at a time as fit.
+    const size_t room = (size_t)(nx + ny) * ntrans;
+    const bool fits = pw.size() <= room;
     size_t chunk = c->mem.limit ? 1 : std::max<size_t>(1, std::min(total, ((size_t)512 << 20) / ibytes));
-    if (chunk > 1 && c->tmpw.ensure(ibytes * chunk + (ndf > 1 ? sizeof(double) * ndf : 0)) != cudaSuccess) {
+    if (chunk > 1 && c->tmpw.ensure(ibytes * chunk + (fits ? 0 : sizeof(double) * pw.size())) != cudaSuccess) {
         cudaGetLastError();
         chunk = 1;
     }
     if (chunk == 1) CUDA_TRY(c, c->tmpw.ensure(ibytes));
     float2 *tmp = (float2 *)c->tmpw.p;
-    double *dpw = (double *)(tmp + n2 * chunk);
-    const bool many = chunk > 1 && ndf > 1;  // weights on the device, copied before anything runs
-    if (many) CUDA_TRY(c, cudaMemcpyAsync(dpw, pw.data(), sizeof(double) * ndf, cudaMemcpyHostToDevice, c->stream));
-    SliceTables st;
-    if ((rc = build_slice_tables(c, g, o, ntrans, dz, st))) return rc;
-    float2 *twr = twiddles(c, ny), *twc = twiddles(c, nx);
-    if (!twr || !twc) return fail(c, MSL_E_NOMEM, "twiddle table allocation failed");
     for (int s = 0; s < nslice; ++s) {
         const int l = seq[s];
         int rf = msl::ROW_TRANS | msl::ROW_FWD;
@@ -546,6 +547,18 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
         ColArgs ca = col_args(g, st, twc, l, w, batch, cf, c->dflag);
         LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, c->stream, c->nsm, &c->launches); }));
     }
+    const bool all = fits || chunk > 1;
+    double *dpw = all && !fits ? (double *)(tmp + n2 * chunk) : (double *)st.d_prop;
+    size_t have = 0, have_end = 0;  // the weights that are there
+    auto weights = [&](size_t j0, size_t j1) -> int {
+        if (j0 >= have && j1 <= have_end) return MSL_OK;
+        have = j0;
+        have_end = all ? pw.size() : std::min(pw.size(), j0 + room);
+        CUDA_TRY(c, cudaMemcpyAsync(dpw, pw.data() + have, sizeof(double) * (have_end - have), cudaMemcpyHostToDevice,
+                                    c->stream));
+        return MSL_OK;
+    };
+    if ((rc = weights(0, 1))) return rc;
     const float kob = (float)lens->k_obj;
     msl::CtfParams cp;
     cp.lam = msl_wavelength(o->kev);
@@ -566,25 +579,23 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
     // three launches each (13 angles x 11 defocus values at 256^2: 1.6 ms, now 0.2).
     for (size_t i0 = 0; i0 < total; i0 += chunk) {
         const int n = (int)std::min(chunk, total - i0);
+        const size_t j0 = i0 % ndf;
+        if (!all && (rc = weights(j0, j0 + 1))) return rc;
         ColArgs ca = col_args(g, st, twc, 0, tmp, n, msl::COL_LOAD | msl::COL_CTF | msl::COL_INV | msl::COL_STORE,
                               c->dflag);
         // image 0 of the pass is i0: start at its spectrum
         ca.in = w + (i0 / ndf) * n2;
         ca.ctf = ctf;
         ca.fan = ndf;
-        ca.img0 = (int)(i0 % ndf);
+        ca.img0 = (int)j0;
         LAUNCH_TRY(c, timed(c, MSL_PROF_COL, [&] { return msl::launch_col_pass(nx, ca, c->stream, c->nsm, &c->launches); }));
         RowArgs r = row_args(g, twr, nullptr, tmp, n, msl::ROW_LOAD | msl::ROW_INV | msl::ROW_ACCUM | msl::ROW_NOSTORE,
                              c->dflag);
         r.accum = img_d;
         r.nimg = n;
-        r.img0 = (int)(i0 % ndf);
-        if (many) {
-            r.accum_wt = dpw;
-            r.nw = ndf;
-        } else {
-            r.accum_w = pw[i0 % ndf];
-        }
+        r.img0 = all ? (int)j0 : (int)(j0 - have);
+        r.accum_wt = dpw;
+        r.nw = all ? ndf : (int)(have_end - have);
         LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
     }
     if (want_exit || exit_d) {  // exit waves: inverse transforms of the spectra in place
@@ -595,7 +606,9 @@ int ctem_core(msl_ctx *c, const msl_grid *g, const msl_optics *o, const float2 *
                                  msl::ROW_LOAD | msl::ROW_INV | msl::ROW_ACCUM | msl::ROW_NOSTORE, c->dflag);
             r.accum = exit_d;
             r.nimg = batch;
-            r.accum_w = weight;
+            if ((rc = weights(ndf, ndf + 1))) return rc;
+            r.accum_wt = dpw + (ndf - have);
+            r.nw = 1;
             LAUNCH_TRY(c, timed(c, MSL_PROF_ROW, [&] { return msl::launch_row_pass(ny, r, c->stream, c->nsm, &c->launches); }));
         }
         if (want_exit) {

@@ -72,12 +72,10 @@ struct RowArgs {
     float scale;           // multiplies the output when != 1
     int *err;              // set to 1 when a bounded wait gives up (may be null)
     // images onto one accumulator (ROW_LOAD [| ROW_INV] | ROW_ACCUM | ROW_NOSTORE): image i
-    // of nimg adds its weight * |psi|^2 to accum[nx][ny], in order: accum_wt[(img0 + i) % nw],
-    // or accum_w for all of them (nw = 0)
+    // of nimg adds accum_wt[(img0 + i) % nw] * |psi|^2 to accum[nx][ny], in order
     double *accum;
     int nimg, img0, nw;
     const double *accum_wt;
-    double accum_w;
     const float2 *const *trans_b;  // per-image transmission rows (replaces trans when set)
     bool shared;           // other streams' kernels run beside this one
 };

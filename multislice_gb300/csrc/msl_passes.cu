@@ -119,13 +119,10 @@ __device__ __forceinline__ float2 phase_grating(float x, float s_hi, float s_lo)
     return make_float2(cn, sn);
 }
 
-__device__ __forceinline__ double image_weight(const RowArgs &a, int img) {
-    return a.nw ? a.accum_wt[(a.img0 + img) % a.nw] : a.accum_w;
-}
 // One image's share of a row's running sums; acc: this thread's first element.
 template <int T, int E>
 __device__ __forceinline__ void add_image(double (&sum)[E], const float2 (&v)[E], const RowArgs &a, int img, double *acc) {
-    const double w = image_weight(a, img);
+    const double w = a.accum_wt[(a.img0 + img) % a.nw];
     if (img == 0) {
 #pragma unroll
         for (int e = 0; e < E; ++e) sum[e] = acc[T * e];
@@ -1323,9 +1320,6 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
             if (lane == 0 && r + 1 < rounds) issue(r + 1);
             const bool mine = r * W + warp < a.nimg;
             bool got = true;
-            double wt[W];  // the round's weights, fetched while its lines are transformed
-#pragma unroll
-            for (int q = 0; q < W; ++q) wt[q] = r * W + q < a.nimg ? image_weight(a, r * W + q) : 0.0;
             if (mine) {
                 float2 *buf = ring + (used & 1u) * UNIT + h * N;
                 got = mbar_wait_bounded(&bar[used & 1u], (used >> 1) & 1u, kWaitLimit);
@@ -1352,11 +1346,12 @@ __global__ void __launch_bounds__(RowTwoCfg<P>::THREADS, 2) row_images_kernel(Ro
             for (int q = 0; q < W; ++q) {
                 const int img = r * W + q;
                 if (img < a.nimg) {
+                    const double w = a.accum_wt[(a.img0 + img) % a.nw];
                     const float2 *x = rings + ((size_t)q * 2 + ((done * ((a.nimg - q + W - 1) / W) + r) & 1)) * UNIT;
 #pragma unroll
                     for (int i = 0; i < PX; ++i) {
                         const float2 v = x[tid + Cfg::THREADS * i];
-                        sum[i] += wt[q] * ((double)v.x * v.x + (double)v.y * v.y);
+                        sum[i] += w * ((double)v.x * v.x + (double)v.y * v.y);
                     }
                 }
             }
