@@ -1794,13 +1794,18 @@ static bool col_maps(const ColArgs &a, int n, int c, int boxr, CUtensorMap *load
 // Whether the two-stage columns of a side overlap at all, three CTAs an SM with a few
 // tiles each.  A plain launch gives every SM one CTA, then a second and a third, so a last
 // round that only some CTAs have is spread over all SMs; as dependents the CTAs go where
-// there is room first, and past one an SM the last round's pile up there.  From some
-// rounds on (13 of 384, 5 of 768) its share no longer matters; below two the overlapped
-// start gains more.  Overlapped against plain, a slice step, by rounds:
+// the row pass leaves room first, and past one an SM the last round's pile up there.  On
+// square grids, whose rows are the two-stage kernel's, its share no longer matters from
+// some rounds on (13 of 384, 5 of 768), and below two the overlapped start gains more.
+// Overlapped against plain, a slice step, by rounds:
 //   384:  1.89 - 5 %, 2.53 + 8 %, 4.63 + 16 %, 5.05 - 4 %, 5.16 + 4 %, 5.47 + 20 %, 6.32 - 4 %, 6.42 + 10 %,
 //         8.21 - 3 %, 8.42 + 16 %, 9.05 - 2 %, 10.74 + 4 %, 12.21 - 2 %, 12.74 + 2 %, 15.2 - 2 %, 27 - 1 %
 //   768:  1.68 - 1 %, 2.11 + 8 %, 3.37 + 8 %, 4.21 - 5 %, 4.63 + 8 %, 5.05 - 4 %, 5.47 - 4 %, 9.26 - 2 %
-static bool mixed_overlaps(int tiles, int ctas, int nsm, int n) {
+// On others which rounds lose (8 to 20 %) and which gain (2 to 6 %) depends on the row
+// pass: at 384 most do (x 128: all from 2 to 13 rounds), so past 20 MB of waves they are
+// launched plainly; at 768 fewer do (x 256, x 2048: none past three rounds).
+static bool mixed_overlaps(const ColArgs &a, int tiles, int ctas, int nsm, int n) {
+    if (a.ny != n) return n == 768 || sizeof(float2) * a.batch * a.ny * n <= (size_t)20 << 20;
     const int rounds = tiles / ctas;
     if (rounds < 2 || rounds >= (n == 384 ? 13 : 5)) return true;
     return rounds >= (n == 384 ? 6 : 4) && tiles % ctas <= nsm;
@@ -1817,7 +1822,7 @@ template <int N> static cudaError_t col_mixed_launch(const ColArgs &a, cudaStrea
     if (!col_maps(a, N, Cfg::C, Cfg::BOXR, &map, &mapo)) return cudaErrorInvalidValue;
     const int ntiles = a.batch * (a.ny / Cfg::C);
     const int grid = nsm * per_sm < ntiles ? nsm * per_sm : ntiles;
-    const bool alone = col_overlaps(a, N) && mixed_overlaps(ntiles, nsm * per_sm, nsm, N);
+    const bool alone = col_overlaps(a, N) && mixed_overlaps(a, ntiles, nsm * per_sm, nsm, N);
     return launch_pass(col_mixed_kernel<N>, grid, Cfg::THREADS, Cfg::SMEM, s, alone, map, mapo, a);
 }
 

@@ -13,10 +13,19 @@ pytestmark = pytest.mark.gpu
                                      (384, 124), (768, 4), (768, 5), (768, 9), (768, 10), (768, 11), (768, 12), (768, 71), (768, 72), (256, 2047),
                                      (256, 2048), (1024, 40), (1024, 41)])
 def test_batches_on_both_sides_of_the_rounds(n, batch):
+    _check(n, n, batch)
+
+
+@pytest.mark.parametrize("nx,ny,batch", [(384, 128, 53), (384, 128, 54), (384, 2048, 3), (384, 2048, 4), (768, 128, 36)])
+def test_rectangles(nx, ny, batch):
+    _check(nx, ny, batch)
+
+
+def _check(n, ny, batch):
     from multislice_gb300 import Context
     g = torch.Generator(device="cuda").manual_seed(n + batch)
-    trans = torch.exp(0.2j * torch.randn(2, n, n, generator=g, device="cuda")).to(torch.complex64)
-    many = torch.exp(0.1j * torch.randn(batch, n, n, generator=g, device="cuda")).to(torch.complex64)
+    trans = torch.exp(0.2j * torch.randn(2, n, ny, generator=g, device="cuda")).to(torch.complex64)
+    many = torch.exp(0.1j * torch.randn(batch, n, ny, generator=g, device="cuda")).to(torch.complex64)
     some = [0, batch // 2, batch - 1]
     ones = [many[b : b + 1].clone() for b in some]
     seq = np.array([0, 1, 1, 0], np.int32)
