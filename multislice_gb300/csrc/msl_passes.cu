@@ -693,7 +693,14 @@ __global__ void __launch_bounds__(ColHalfCfg<L>::THREADS, 1)
 template <int N> __device__ __forceinline__ void mixed_tables(float2 *t, const float2 *__restrict__ tw) {
     constexpr int RB = Mixed<N>::RB;
     tw += Mixed<N>::GTW_OFF;
-    for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) t[i] = tw[i < N ? i : (i - N) % 24 * RB + (i - N) / 24];
+    float2 v[2 * N / 128];  // of 128 threads, every load in flight at once
+#pragma unroll
+    for (int j = 0; j < 2 * N / 128; ++j) {
+        const int i = threadIdx.x + 128 * j;
+        v[j] = tw[i < N ? i : (i - N) % 24 * RB + (i - N) / 24];
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * N / 128; ++j) t[threadIdx.x + 128 * j] = v[j];
 }
 
 // ---------------------------------------- two-stage column pass, 384 and 768
@@ -713,7 +720,7 @@ template <int N> struct ColMixedCfg {
     static constexpr size_t OFF_T = 2 * SLOT, OFF_RED = OFF_T + sizeof(float2) * 2 * N;
     static constexpr size_t OFF_BAR = OFF_RED + sizeof(double) * NWARP * kMaxDet;
     static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * 2 + 128;
-    static_assert(BOXR <= 256 && BOXR * NBOX == N && SLOT % 128 == 0, "TMA boxes tile the column");
+    static_assert(BOXR <= 256 && BOXR * NBOX == N && SLOT % 128 == 0 && THREADS == 128, "TMA boxes tile the column");
 };
 
 template <int N>
@@ -973,6 +980,7 @@ template <int N> struct RowMixedCfg {
     static constexpr size_t SMEM = OFF_BAR + sizeof(uint64_t) * W * 2 + 128;  // + base alignment
     static_assert(sizeof(float2) * M::SLOTS % 16 == 0 && (LPW == 1 || M::SLOTS % 16 == 8),
                   "bulk copies land on 16 bytes; a second line shifts by half the banks");
+    static_assert(THREADS == 128, "mixed_tables");
 };
 template <int N, bool IMG>
 __global__ void __launch_bounds__(RowMixedCfg<N>::THREADS, IMG ? 1 : RowMixedCfg<N>::MINB) row_mixed_kernel(RowArgs a) {
