@@ -78,6 +78,11 @@ struct TripleSum {
         e = two_sum(mid, e);
         lo = __fadd_rn(lo, e);
     }
+    __device__ __forceinline__ void add(const float *p, int stride) {  // another such sum
+        add(p[0]);
+        lo = __fadd_rn(lo, two_sum(mid, p[stride]));
+        lo = __fadd_rn(lo, p[2 * stride]);
+    }
     // NaN where a sum on the way overflowed (or a value was no number)
     __device__ __forceinline__ double value() const { return ((double)lo + (double)mid) + (double)hi; }
 };
@@ -907,12 +912,14 @@ __global__ void __launch_bounds__(32 * kEdgeWarps)
 // the complex parameters: the expanded layer holds [[Wr, -Wi], [Wi, Wr]], so dWr is
 // the sum of its two Wr blocks and dWi the difference of the others; db likewise.
 // 32 parameters a block, their partials shared among kRedParts threads each (one
-// thread over all of them waited for its loads: 105 us for 152 CTAs; FP64 sums took
-// 33, three-float ones 19).
+// thread over all of them waited for its loads: 105 us for 152 CTAs of 64 x 64 channels,
+// now 12.5), then each of a parameter's four sums a warp's.  The six of a gradient step
+// of 8 waves of 256^2 take 15 us on average; 33 with FP64 sums.
 constexpr int kRedParts = 16;
 __global__ void __launch_bounds__(32 * kRedParts)
     dw_reduce_kernel(const float *__restrict__ partial, int nblocks, int co, int ci, float *__restrict__ g) {
     __shared__ float part[kRedParts][4][3][32];
+    __shared__ double sums[4][32];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, nw = 9 * co * ci, idx = blockIdx.x * 32 + lane;
     const bool live = idx < nw + co, isb = idx >= nw;
     const int tap = isb ? 9 : idx / (co * ci), o = isb ? idx - nw : (idx / ci) % co, i = isb ? 0 : idx % ci;
@@ -934,20 +941,20 @@ __global__ void __launch_bounds__(32 * kRedParts)
         part[grp][j][2][lane] = ps[j].lo;
     }
     __syncthreads();
-    if (grp == 0 && live) {
-        double s[4];
+    if (grp < 4 && live) {  // a warp a sum
+        TripleSum t;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int q = 1; q < kRedParts; ++q)
-#pragma unroll
-                for (int i = 0; i < 3; ++i) ps[j].add(part[q][j][i][lane]);
-            s[j] = ps[j].value();
-            if (!isfinite(s[j])) {  // beyond float's range on the way: FP64 has room
-                s[j] = 0.0;
-                for (int b = 0; b < nblocks; ++b) s[j] += partial[((size_t)b * 10 + tap) * 64 * 64 + at[j]];
-            }
+        for (int q = 0; q < kRedParts; ++q) t.add(&part[q][grp][0][lane], 32);
+        double v = t.value();
+        if (!isfinite(v)) {  // beyond float's range on the way: FP64 has room
+            v = 0.0;
+            for (int b = 0; b < nblocks; ++b) v += partial[((size_t)b * 10 + tap) * 64 * 64 + at[grp]];
         }
+        sums[grp][lane] = v;
+    }
+    __syncthreads();
+    if (grp == 0 && live) {
+        const double s[4] = {sums[0][lane], sums[1][lane], sums[2][lane], sums[3][lane]};
         float *out = g + (size_t)2 * idx;  // weights [tap][o][i][2], then bias [o][2]
         out[0] = (float)s[0] + (isb ? 0.f : (float)s[1]);
         out[1] = (float)s[2] - (isb ? 0.f : (float)s[3]);
